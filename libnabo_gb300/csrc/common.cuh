@@ -12,7 +12,7 @@
 //                meta high 27 bits = right-child index (inner) or bucket
 //                                    size (leaf)
 //              f32: {meta, cut | bucketStart}            8 bytes
-//              f64: {meta, bucketStart, cut}            16 bytes
+//              f64: {meta, bucketStart | (float)cut, cut} 16 bytes
 #pragma once
 
 #include <cuda_runtime.h>
@@ -123,7 +123,7 @@ template <>
 __device__ __forceinline__ void store_inner<double>(Node<double>* n, uint32_t cd, uint32_t right, double cut) {
   Node<double> v;
   v.meta = make_meta(cd, right);
-  v.start = 0;
+  v.start = __float_as_uint((float)cut);
   v.cut = cut;
   *n = v;
 }
@@ -146,6 +146,8 @@ __device__ __forceinline__ void store_leaf<double>(Node<double>* n, uint32_t cou
 }
 __device__ __forceinline__ uint32_t node_start(const Node<float>& n) { return n.start; }
 __device__ __forceinline__ uint32_t node_start(const Node<double>& n) { return n.start; }
+// an inner double node's cut rounded to float (for the search's float bounds)
+__device__ __forceinline__ float node_cut_float(const Node<double>& n) { return __uint_as_float(n.start); }
 
 __device__ __forceinline__ Node<float> load_node(const Node<float>* __restrict__ nodes, uint32_t i) {
   const uint2 v = __ldg(reinterpret_cast<const uint2*>(nodes) + i);

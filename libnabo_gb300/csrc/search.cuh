@@ -89,19 +89,18 @@ struct TopK {
 };
 
 // double lists of 16 or more entries in the kd-tree search: a binary
-// max-heap of (dist2 bits, index) in shared memory, slot-major with one
-// column per thread (blocks of at most kHeapThreads threads), the root kept
-// in registers for the accept test. Held in registers, such a list (3
+// max-heap of (dist2 bits, index) in (dynamic) shared memory, a section per
+// warp, slot-major with one column per lane, the root kept in registers for
+// the accept test. Held in registers, such a list (3
 // registers an entry) spilled under the search kernel's register cap, and
 // every insertion walked the spilled entries through local memory (8-D,
 // k = 32: 2.2 G local loads a launch). Here an insertion sifts down at most
 // log2(k) levels. The entries and their order are those of TopK: the k
 // smallest (dist2, index) pairs, empty entries (+inf, -1), written out in
 // ascending order.
-constexpr int kHeapThreads = 128;
 template <int K>
 struct SmemTopK {
-  unsigned long long* d;  // entry j of this thread's list at d[j * kHeapThreads]
+  unsigned long long* d;  // entry j of this thread's list at d[j * 32]
   int* ix;
   int n;
   unsigned long long rootD;
@@ -113,16 +112,16 @@ struct SmemTopK {
     return (unsigned long long)__double_as_longlong(x);
   }
   __device__ __forceinline__ void init(int k) {
-    __shared__ unsigned long long sd[K * kHeapThreads];
-    __shared__ int si[K * kHeapThreads];
-    d = sd + threadIdx.x;
-    ix = si + threadIdx.x;
+    extern __shared__ __align__(16) unsigned char heapSmem[];
+    const int column = (threadIdx.x >> 5) * K * 32 + (threadIdx.x & 31);
+    d = reinterpret_cast<unsigned long long*>(heapSmem) + column;
+    ix = reinterpret_cast<int*>(heapSmem + (size_t)blockDim.x * K * sizeof(unsigned long long)) + column;
     n = k < K ? k : K;
     rootD = bits(Ar<double>::inf());
     rootI = -1;
     for (int j = 0; j < n; ++j) {
-      d[j * kHeapThreads] = rootD;
-      ix[j * kHeapThreads] = -1;
+      d[j * 32] = rootD;
+      ix[j * 32] = -1;
     }
   }
   __device__ __forceinline__ double head() const { return __longlong_as_double((long long)rootD); }
@@ -135,11 +134,11 @@ struct SmemTopK {
       const int l = 2 * j + 1;
       if (l >= m) break;
       int c = l;
-      unsigned long long cd = d[l * kHeapThreads];
-      int ci = ix[l * kHeapThreads];
+      unsigned long long cd = d[l * 32];
+      int ci = ix[l * 32];
       if (l + 1 < m) {
-        const unsigned long long rd = d[(l + 1) * kHeapThreads];
-        const int ri = ix[(l + 1) * kHeapThreads];
+        const unsigned long long rd = d[(l + 1) * 32];
+        const int ri = ix[(l + 1) * 32];
         if (greater(rd, ri, cd, ci)) {
           c = l + 1;
           cd = rd;
@@ -147,12 +146,12 @@ struct SmemTopK {
         }
       }
       if (!greater(cd, ci, x, xi)) break;
-      d[j * kHeapThreads] = cd;
-      ix[j * kHeapThreads] = ci;
+      d[j * 32] = cd;
+      ix[j * 32] = ci;
       j = c;
     }
-    d[j * kHeapThreads] = x;
-    ix[j * kHeapThreads] = xi;
+    d[j * 32] = x;
+    ix[j * 32] = xi;
   }
   // Drops the largest entry and inserts (dist, idx); requires accepts(dist, idx).
   __device__ __forceinline__ void insert(double dist, int idx) {
@@ -162,7 +161,7 @@ struct SmemTopK {
   }
   __device__ __forceinline__ int count(int) const {
     int c = 0;
-    for (int j = 0; j < n; ++j) c += ix[j * kHeapThreads] >= 0 ? 1 : 0;
+    for (int j = 0; j < n; ++j) c += ix[j * 32] >= 0 ? 1 : 0;
     return c;
   }
   // Writes the entries in ascending order (the largest last), emptying the
@@ -175,7 +174,7 @@ struct SmemTopK {
       oi[m - 1] = ti;
       od[m - 1] = __longlong_as_double((long long)top);
       found += ti >= 0 ? 1 : 0;
-      if (m > 1) sift(d[(m - 1) * kHeapThreads], ix[(m - 1) * kHeapThreads], m - 1);
+      if (m > 1) sift(d[(m - 1) * 32], ix[(m - 1) * 32], m - 1);
     }
     return found;
   }
@@ -191,10 +190,14 @@ struct SmemTopK {
 template <typename T, int K>
 struct SearchHeap {
   using type = TopK<T, K>;
+  static constexpr size_t bytes(int) { return 0; }  // dynamic shared memory of a block
 };
 template <int K>
 struct SearchHeap<double, K> {
   using type = std::conditional_t<(K >= 16), SmemTopK<K>, TopK<double, K>>;
+  static constexpr size_t bytes(int threads) {
+    return K >= 16 ? (size_t)threads * K * (sizeof(unsigned long long) + sizeof(int)) : 0;
+  }
 };
 
 // float: one 64-bit key per entry, (bit pattern of dist2) << 32 | index.
@@ -264,13 +267,49 @@ struct TopK<float, K> {
   }
 };
 
+// Distances and box distances as values that order like them. A float is its
+// own key. Doubles compare as bit patterns on the integer pipe: GB300 runs
+// FP64 at 1/64 of the FP32 rate, and a DSETP takes an FP64 slot like the
+// arithmetic. They are never negative (a box distance only grows along a
+// path: a cell's cut lies no further out than the cell's own face, so
+// -(old^2) + new^2 >= 0 in round-to-nearest too), where the pattern orders
+// like the value, and a NaN of either sign is above every number.
+__device__ __forceinline__ float dist_key(float x) { return x; }
+__device__ __forceinline__ unsigned long long dist_key(double x) { return (unsigned long long)__double_as_longlong(x); }
+// x <= limit(b) iff x <= b; limit(NaN) admits nothing.
+__device__ __forceinline__ float dist_limit(float b) { return b; }
+__device__ __forceinline__ unsigned long long dist_limit(double b) {
+  const unsigned long long k = dist_key(b);
+  return k <= 0x7ff0000000000000ull ? k + 1ull : 0ull;
+}
+__device__ __forceinline__ bool within(float x, float limit) { return x <= limit; }
+__device__ __forceinline__ bool within(double x, unsigned long long limit) { return dist_key(x) < limit; }
+// The smaller limit, where a NaN second argument (a radius) wins.
+__device__ __forceinline__ float min_limit(float head, float radius) { return head < radius ? head : radius; }
+__device__ __forceinline__ unsigned long long min_limit(unsigned long long head, unsigned long long radius) {
+  return head < radius ? head : radius;
+}
+// x > 0; false for NaN
+__device__ __forceinline__ bool positive(float x) { return x > 0.0f; }
+__device__ __forceinline__ bool positive(double x) { return dist_key(x) - 1ull < 0x7ff0000000000000ull; }
+
+// v[c]: a select per entry, or for 8 and 16 entries a tree of selects on the
+// bits of c (half the predicates).
 template <typename T, int D>
 __device__ __forceinline__ T pick(const T (&v)[D], int c) {
-  T r = v[0];
+  if constexpr (D == 8 || D == 16) {
+    T h[D / 2];
+    const bool odd = c & 1;
 #pragma unroll
-  for (int d = 1; d < D; ++d)
-    if (c == d) r = v[d];
-  return r;
+    for (int d = 0; d < D / 2; ++d) h[d] = odd ? v[2 * d + 1] : v[2 * d];
+    return pick(h, c >> 1);
+  } else {
+    T r = v[0];
+#pragma unroll
+    for (int d = 1; d < D; ++d)
+      if (c == d) r = v[d];
+    return r;
+  }
 }
 
 template <typename T, int D>
@@ -307,7 +346,7 @@ __global__ void k_leaf_cells(const Node<T>* __restrict__ nodes, const T* __restr
     const Node<T> nd = load_node(nodes, node);
     if (node_is_leaf(nd.meta)) break;
     const T newOff = Ar<T>::sub(pick(q, (int)node_dim(nd.meta)), nd.cut);
-    node = newOff > T(0) ? node_payload(nd.meta) : node + 1;
+    node = positive(newOff) ? node_payload(nd.meta) : node + 1;
   }
   cell[i] = node;
   if (hist) rank[i] = atomicAdd(hist + node, 1u);
@@ -388,7 +427,8 @@ struct KnnLaunch {
 // subtraction errors are at most 2.1 * 2^-24 * (|q| + |p|) each), so
 //     LB = sum_d max(0, |q~_d - p~_d| - e)^2,  taken * (1 - 2^-17)
 // is below the exact squared distance, float roundings of LB itself and the
-// double sum's own rounding included. A point with LB above a float at or
+// double sum's own rounding included (less 2^-140, for squares that underflow).
+// A point with LB above a float at or
 // above min(head, maxRadius^2) cannot enter the heap, and only the others
 // get the exact double distance: results are unchanged. Coordinates beyond
 // the float range make e infinite, which rejects nothing.
@@ -419,9 +459,10 @@ struct LeafFilter<double, D> {
     }
   }
   __device__ __forceinline__ bool on() const { return recs32 != nullptr; }
-  // a float at or above min(head, maxRadius2)
+  // a float at or above min(head, maxRadius2) (a NaN radius: head)
   __device__ __forceinline__ float threshold(double head, double maxRadius2) const {
-    return __double2float_ru(fmin(head, maxRadius2));
+    const unsigned long long h = dist_key(head), r = dist_key(maxRadius2);
+    return __double2float_ru(__longlong_as_double((long long)(r < h ? r : h)));
   }
   __device__ __forceinline__ bool rejects(int64_t i, float thr) const {
     Rec<float, D> f;
@@ -432,7 +473,7 @@ struct LeafFilter<double, D> {
       const float a = fmaxf(fabsf(qf[d] - f.p.c[d]) - e, 0.0f);
       lb += a * a;
     }
-    return lb * (1.0f - 0x1p-17f) > thr;
+    return fmaf(lb, 1.0f - 0x1p-17f, -0x1p-140f) > thr;
   }
 };
 
@@ -478,6 +519,8 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
       T dj[kChunk];
       int ij[kChunk];
       const float thr = flt.on() ? flt.threshold(heap.head(), maxRadius2) : 0.0f;
+      const auto radLimit = dist_limit(maxRadius2);
+      const auto minKey = dist_key(Ar<T>::eps());
 #pragma unroll
       for (int j = 0; j < kChunk; ++j) {
         dj[j] = Ar<T>::inf();
@@ -487,7 +530,8 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
           load_rec(recs, (int64_t)st + base + j, r);
           dj[j] = dist2_seq(q, r);
           ij[j] = r.p.idx;
-          const bool ok = want && dj[j] <= maxRadius2 && heap.accepts(dj[j], ij[j]) && dj[j] > minDist;
+          const bool ok = want && within(dj[j], radLimit) && heap.accepts(dj[j], ij[j]) &&
+                          (minDist < T(0) || dist_key(dj[j]) > minKey);
           mask |= ok ? (1u << j) : 0u;
         }
       }
@@ -566,7 +610,8 @@ __device__ __forceinline__ void scan_first_leaf(const Rec<float, D>* __restrict_
   if (cnt > (uint32_t)B) scan_leaf<float, D, K>(recs, st + B, cnt - B, q, maxRadius2, minDist, want, heap, flt);
 }
 
-// A pushed far child as 32-bit words [rd | off[0..D-1] | node] (a T is one
+// A pushed far child as 32-bit words [rd | off2[0..D-1] | node] (off2: the
+// squared offsets, all the box-distance update needs; a T is one
 // word for float, two for double) in 16-byte chunks: a push is one 128-bit
 // local store per chunk (a lone trailing word is stored alone), a pop reads
 // the first chunk, which holds rd, and the rest only if the child is
@@ -597,7 +642,7 @@ __device__ __forceinline__ double get_t<double>(const uint32_t* w, int i) {
 }
 
 template <typename T, int D>
-__device__ __forceinline__ void stack_push(StackRec<T, D>& e, T rd, const T (&off)[D], int cd, T newOff,
+__device__ __forceinline__ void stack_push(StackRec<T, D>& e, T rd, const T (&off2)[D], int cd, T new2,
                                            uint32_t node) {
   using R = StackRec<T, D>;
   uint32_t w[R::kChunks * 4];
@@ -605,7 +650,7 @@ __device__ __forceinline__ void stack_push(StackRec<T, D>& e, T rd, const T (&of
   for (int i = 0; i < R::kChunks * 4; ++i) w[i] = 0u;
   put_t(w, 0, rd);
 #pragma unroll
-  for (int d = 0; d < D; ++d) put_t(w, R::kTW * (1 + d), d == cd ? newOff : off[d]);
+  for (int d = 0; d < D; ++d) put_t(w, R::kTW * (1 + d), d == cd ? new2 : off2[d]);
   w[R::kNode] = node;
 #pragma unroll
   for (int c = 0; c < R::kChunks; ++c) {
@@ -624,7 +669,7 @@ __device__ __forceinline__ T stack_rd(const StackRec<T, D>& e) {
 }
 
 template <typename T, int D>
-__device__ __forceinline__ uint32_t stack_take(const StackRec<T, D>& e, T (&off)[D]) {
+__device__ __forceinline__ uint32_t stack_take(const StackRec<T, D>& e, T (&off2)[D]) {
   using R = StackRec<T, D>;
   uint32_t w[R::kChunks * 4];
 #pragma unroll
@@ -641,7 +686,7 @@ __device__ __forceinline__ uint32_t stack_take(const StackRec<T, D>& e, T (&off)
     }
   }
 #pragma unroll
-  for (int d = 0; d < D; ++d) off[d] = get_t<T>(w, R::kTW * (1 + d));
+  for (int d = 0; d < D; ++d) off2[d] = get_t<T>(w, R::kTW * (1 + d));
   return w[R::kNode];
 }
 
@@ -661,6 +706,59 @@ struct SlabStack {
   __device__ __forceinline__ StackRec<T, D>& operator[](int sp) { return base[(int64_t)sp * stride]; }
 };
 
+// What the thread at order position t searches.
+template <typename T>
+struct QueryTask {
+  int64_t qi;       // query
+  int64_t outBase;  // its first result entry
+  int k;
+  uint32_t root;
+  T maxRadius2;
+  // a bounded search (per-query radius) that misses may run once more
+  // without its bound (the learned-radius form's fallback)
+  bool mayFall;
+};
+
+template <typename T>
+__device__ __forceinline__ QueryTask<T> query_task(const KnnLaunch& a, int64_t t) {
+  QueryTask<T> w;
+  w.k = a.k;
+  w.root = 0;
+  if (a.runPrefix) {
+    const int64_t g = a.runPrefix[a.runBegin] + t;
+    int lo = a.runBegin, hi = a.runEnd - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (a.runPrefix[mid] <= g)
+        lo = mid;
+      else
+        hi = mid - 1;
+    }
+    const int c = a.runCloud[lo];
+    w.qi = (int64_t)a.order[a.bQueryOffset[c] + (g - a.runPrefix[lo])];
+    w.k = a.bK[c];
+    w.root = (uint32_t)a.bNodeOffset[c];
+    w.outBase = a.bOutOffset[c] + (w.qi - a.bQueryOffset[c]) * (int64_t)w.k;
+  } else {
+    w.qi = a.order ? (int64_t)a.order[t] : t;
+    w.outBase = w.qi * (int64_t)a.k;
+    if (a.bQueryOffset) {
+      const int c = cloud_of(a.bQueryOffset, a.bClouds, w.qi);
+      w.k = a.bK[c];
+      w.root = (uint32_t)a.bNodeOffset[c];
+      w.outBase = a.bOutOffset[c] + (w.qi - a.bQueryOffset[c]) * (int64_t)w.k;
+    }
+  }
+  w.maxRadius2 = (T)a.maxRadius2;
+  w.mayFall = false;
+  if (a.maxRadii) {
+    const T r = static_cast<const T*>(a.maxRadii)[w.qi];
+    w.maxRadius2 = Ar<T>::mul(r, r);
+    w.mayFall = a.fallbackRadius >= 0.0 && (double)r < a.fallbackRadius;
+  }
+  return w;
+}
+
 // One query (order position t) in the reference's visit order, structured
 // descend / leaf / pop so the lanes of a warp run each phase together: all
 // lanes descend until every lane stands on a leaf, then all scan their
@@ -679,78 +777,50 @@ __device__ __forceinline__ void knn_query(const KnnLaunch& a, int64_t t, S& stk,
   const Rec<T, D>* __restrict__ recs = static_cast<const Rec<T, D>*>(a.recs);
   const T* __restrict__ query = static_cast<const T*>(a.query);
   uint32_t touched = 0;  // a query touches at most the cloud's n < 2^31 points
-  int64_t qi;
-  int k = a.k;
-  uint32_t root = 0;
-  int64_t outBase;
-  if (a.runPrefix) {
-    const int64_t g = a.runPrefix[a.runBegin] + t;
-    int lo = a.runBegin, hi = a.runEnd - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.runPrefix[mid] <= g)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
-    const int c = a.runCloud[lo];
-    qi = (int64_t)a.order[a.bQueryOffset[c] + (g - a.runPrefix[lo])];
-    k = a.bK[c];
-    root = (uint32_t)a.bNodeOffset[c];
-    outBase = a.bOutOffset[c] + (qi - a.bQueryOffset[c]) * (int64_t)k;
-  } else {
-    qi = a.order ? (int64_t)a.order[t] : t;
-    outBase = qi * (int64_t)a.k;
-    if (a.bQueryOffset) {
-      const int c = cloud_of(a.bQueryOffset, a.bClouds, qi);
-      k = a.bK[c];
-      root = (uint32_t)a.bNodeOffset[c];
-      outBase = a.bOutOffset[c] + (qi - a.bQueryOffset[c]) * (int64_t)k;
-    }
-  }
+  const QueryTask<T> task = query_task<T>(a, t);
+  const int k = task.k;
   T q[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) q[d] = d < a.dim ? query[qi * a.qStride + d] : T(0);
-  T maxRadius2 = (T)a.maxRadius2;
-  // a bounded search (per-query radius) that misses may run once more
-  // without its bound (the learned-radius form's fallback)
-  bool mayFall = false;
-  if (a.maxRadii) {
-    const T r = static_cast<const T*>(a.maxRadii)[qi];
-    maxRadius2 = Ar<T>::mul(r, r);
-    mayFall = a.fallbackRadius >= 0.0 && (double)r < a.fallbackRadius;
-  }
+  for (int d = 0; d < D; ++d) q[d] = d < a.dim ? query[task.qi * a.qStride + d] : T(0);
+  T maxRadius2 = task.maxRadius2;
+  bool mayFall = task.mayFall;
   const T maxError2 = (T)a.maxError2;
   typename SearchHeap<T, K>::type heap;
   heap.init(k);
   LeafFilter<T, D> flt;
   flt.init(a.recs32, a.coordMax, q);
-  T off[D];
+  // squared offsets to the cell, per dimension: the reference's
+  // rd += -(old*old) + new*new (nabo/kdtree_cpu.cpp:415, 433) reads only
+  // squares, so the product is kept instead of computed again each step
+  T off2[D];
   for (;;) {  // the search, and at most once more without the bound
+    const auto radLimit = dist_limit(maxRadius2);
 #pragma unroll
-    for (int d = 0; d < D; ++d) off[d] = T(0);
+    for (int d = 0; d < D; ++d) off2[d] = T(0);
     int sp = 0;
-    uint32_t node = root;
+    uint32_t node = task.root;
     T rd = T(0);
     bool fresh = true;  // no leaf scanned yet: the top-k is empty
     for (;;) {
       // descend to a leaf, pushing far children
       // min(maxRadius2, head), where a NaN radius (which passes nothing) wins
-      const T bound = EXACT ? (heap.head() < maxRadius2 ? heap.head() : maxRadius2) : T(0);
+      const auto headLimit = dist_limit(heap.head());
+      const auto bound = min_limit(headLimit, radLimit);
       Node<T> nd = load_node(nodes, node);
       while (!node_is_leaf(nd.meta)) {
         const int cd = (int)node_dim(nd.meta);
         const T newOff = Ar<T>::sub(pick(q, cd), nd.cut);
-        const T oldOff = pick(off, cd);
-        const T rdFar = Ar<T>::add(rd, Ar<T>::add(-Ar<T>::mul(oldOff, oldOff), Ar<T>::mul(newOff, newOff)));
+        const T new2 = Ar<T>::mul(newOff, newOff);
+        const T rdFar = Ar<T>::add(rd, Ar<T>::add(-pick(off2, cd), new2));
         const uint32_t right = node_payload(nd.meta);
-        const uint32_t nearN = newOff > T(0) ? right : node + 1;
-        const uint32_t farN = newOff > T(0) ? node + 1 : right;
-        const bool far = EXACT ? rdFar <= bound
-                               : (rdFar <= maxRadius2 && Ar<T>::mul(rdFar, maxError2) <= heap.head());
+        const bool nearRight = positive(newOff);
+        const uint32_t nearN = nearRight ? right : node + 1;
+        const uint32_t farN = nearRight ? node + 1 : right;
+        const bool far = EXACT ? within(rdFar, bound)
+                               : (within(rdFar, radLimit) && within(Ar<T>::mul(rdFar, maxError2), headLimit));
         // sp <= tree height <= cap (checked by the caller); the test only
         // makes the bound explicit
-        if (far && sp < cap) stack_push(stk[sp++], rdFar, off, cd, newOff, farN);
+        if (far && sp < cap) stack_push(stk[sp++], rdFar, off2, cd, new2, farN);
         node = nearN;
         nd = load_node(nodes, node);
       }
@@ -768,12 +838,13 @@ __device__ __forceinline__ void knn_query(const KnnLaunch& a, int64_t t, S& stk,
       touched += cnt;
       // pop the next far child that can still hold a better neighbour
       bool more = false;
+      const auto popLimit = dist_limit(heap.head());
       while (sp > 0) {
         --sp;
         const T e = stack_rd(stk[sp]);
-        if ((EXACT ? e : Ar<T>::mul(e, maxError2)) <= heap.head()) {
+        if (within(EXACT ? e : Ar<T>::mul(e, maxError2), popLimit)) {
           rd = e;
-          node = stack_take(stk[sp], off);
+          node = stack_take(stk[sp], off2);
           more = true;
           break;
         }
@@ -786,8 +857,202 @@ __device__ __forceinline__ void knn_query(const KnnLaunch& a, int64_t t, S& stk,
     heap.init(k);
     if (a.fallbacks) atomicAdd(a.fallbacks, 1);
   }
-  const int f = heap.store(k, a.outIdx + outBase, static_cast<T*>(a.outD2) + outBase);
-  if (a.found) a.found[qi] = f;
+  const int f = heap.store(k, a.outIdx + task.outBase, static_cast<T*>(a.outD2) + task.outBase);
+  if (a.found) a.found[task.qi] = f;
+  touchedOut += touched;
+}
+
+// Double searches with local stacks: the traversal above, with its FP64 work
+// put off until a decision needs it. GB300 runs FP64 at 1/64 of its FP32
+// rate, and with a handful of a warp's lanes active a step's FP64
+// instructions cost as much as with all of them, so what counts is how often
+// a warp executes them.
+//  - The near side is the sign of the float difference of the rounded
+//    coordinates when that exceeds its error bound e (LeafFilter), else of
+//    the double difference.
+//  - A far child is pushed when a float lower bound of its box distance is
+//    within the pruning limit: rd - old^2 + new^2 with rd rounded down, the
+//    old square from its upper 32 bits rounded up and new = |q~ - cut~| - e.
+//    Its error is below 2^-20 of the sum (old^2 and rd are at most the
+//    distance itself), covered by the factor 1 - 2^-17, and 2^-120 covers
+//    underflow. The exact distance, the reference's rounded update
+//    (nabo/kdtree_cpu.cpp:415, 433), is computed when the child is popped
+//    and its lower bound is still within the limit: the reference's
+//    decision, taken with the head the reference has at that point, so the
+//    visits (and TOUCH_STATISTICS) are the same.
+//  - A descent shares one frame (rd and the squared offsets it started
+//    from), written once, instead of a copy per pushed child; an entry is
+//    16 bytes: [far child | cut dimension << 27, lower bound with its low 8
+//    bits replaced by the frame's slot, cut].
+//  - A leaf's points are filtered in float first; the exact distances run in
+//    a loop over the points that passed, so a warp executes them as often as
+//    the lane with the most such points, not once per point some lane needs.
+// (Search kernel, exact distances at every step -> here: 8-D clusters, 200 k
+// points, 50 k queries, k = 32 12.9 -> 9.8 ms; 3-D uniform, 100 k points,
+// 30 k queries, k = 10 302 -> 250 us.)
+template <int D, int STACK>
+struct F64Stack {
+  static constexpr int kPairs = (D + 2) / 2;  // rd and D squares, in pairs
+  uint4 entry[STACK];
+  double2 frame[STACK][kPairs];
+  static_assert(STACK <= 256, "frame slots take 8 bits");
+};
+
+// A float at or above x >= 0 (less 2^-126) and within 2^-20 of it, from x's
+// upper 32 bits; infinity stays.
+__device__ __forceinline__ float upper_bound_of_hi(uint32_t hi) {
+  const int u = (int)hi + 1 - 0x38000000;
+  return hi >= 0x47efffffu ? __int_as_float(0x7f800000) : (u > 0 ? __int_as_float(u << 3) : 0.0f);
+}
+
+template <int D, int K, bool EXACT, int STACK>
+__device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64Stack<D, STACK>& stk,
+                                              uint32_t& touchedOut) {
+  constexpr unsigned long long kEps = 0x3cb0000000000000ull;  // 2^-52, numeric_limits<double>::epsilon()
+  const Node<double>* __restrict__ nodes = static_cast<const Node<double>*>(a.nodes);
+  const Rec<double, D>* __restrict__ recs = static_cast<const Rec<double, D>*>(a.recs);
+  uint32_t touched = 0;
+  const QueryTask<double> task = query_task<double>(a, t);
+  const int k = task.k;
+  const double* __restrict__ query = static_cast<const double*>(a.query) + task.qi * a.qStride;
+  double q[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) q[d] = d < a.dim ? query[d] : 0.0;
+  double maxRadius2 = task.maxRadius2;
+  bool mayFall = task.mayFall;
+  const double maxError2 = a.maxError2;
+  // a float at or above 1 / maxError2 (inf or NaN where that has none: no
+  // child is then left out by its lower bound)
+  const float invError = EXACT ? 1.0f : __double2float_ru(1.0 / maxError2) * (1.0f + 0x1p-20f);
+  typename SearchHeap<double, K>::type heap;
+  heap.init(k);
+  LeafFilter<double, D> flt;
+  flt.init(a.recs32, a.coordMax, q);
+  double off2[D];
+  for (;;) {  // the search, and at most once more without the bound
+    const unsigned long long radLimit = dist_limit(maxRadius2);
+    const bool anyRadius = radLimit != 0ull;  // a NaN radius accepts nothing
+#pragma unroll
+    for (int d = 0; d < D; ++d) off2[d] = 0.0;
+    int sp = 0;
+    uint32_t node = task.root;
+    double rd = 0.0;
+    float rdDown = 0.0f;
+    float leafThr = flt.threshold(heap.head(), maxRadius2);
+    // a float at or above the largest box distance still searched,
+    // min(maxRadius2, head / maxError2)
+    const auto prune_threshold = [&]() {
+      return EXACT ? leafThr
+                   : fminf(__double2float_ru(maxRadius2), __fmul_ru(__double2float_ru(heap.head()), invError));
+    };
+    float pruneThr = prune_threshold();
+    for (;;) {
+      const int frame = sp;
+      bool saved = false;
+      Node<double> nd = load_node(nodes, node);
+      while (!node_is_leaf(nd.meta)) {
+        const int cd = (int)node_dim(nd.meta);
+        const float df = pick(flt.qf, cd) - node_cut_float(nd);
+        const float ad = fabsf(df);
+        bool nearRight = df > 0.0f;
+        if (!(ad > flt.e)) nearRight = positive(Ar<double>::sub(query[cd], nd.cut));
+        const float nf = fmaxf(ad - flt.e, 0.0f);
+        uint32_t hi[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) hi[d] = (uint32_t)__double2hiint(off2[d]);
+        const float low = fmaf((rdDown - upper_bound_of_hi(pick(hi, cd))) + nf * nf, 1.0f - 0x1p-17f, -0x1p-120f);
+        const uint32_t right = node_payload(nd.meta);
+        const uint32_t farN = nearRight ? node + 1 : right;
+        node = nearRight ? right : node + 1;
+        // (a NaN bound, from infinite coordinates, is pushed and decided exactly)
+        if (anyRadius && !(low > pruneThr) && sp < STACK) {
+          if (!saved) {
+            saved = true;
+            double v[2 * F64Stack<D, STACK>::kPairs];
+            v[0] = rd;
+#pragma unroll
+            for (int d = 0; d < D; ++d) v[1 + d] = off2[d];
+            if (D % 2 == 0) v[D + 1] = 0.0;
+#pragma unroll
+            for (int p = 0; p < F64Stack<D, STACK>::kPairs; ++p)
+              stk.frame[frame][p] = make_double2(v[2 * p], v[2 * p + 1]);
+          }
+          const uint32_t lowBits = low > 0.0f ? __float_as_uint(low) : 0u;
+          stk.entry[sp++] =
+              make_uint4(farN | ((uint32_t)cd << 27), (lowBits & ~255u) | (uint32_t)frame,
+                         (uint32_t)__double2loint(nd.cut), (uint32_t)__double2hiint(nd.cut));
+        }
+        nd = load_node(nodes, node);
+      }
+      // leaf
+      const uint32_t cnt = node_payload(nd.meta);
+      const uint32_t st = node_start(nd);
+      touched += cnt;
+      bool changed = false;
+      for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t m = cnt - base < 32u ? cnt - base : 32u;
+        unsigned mask = 0;
+        for (uint32_t j0 = 0; j0 < m; j0 += 4) {
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j)
+            if (j0 + j < m && !flt.rejects((int64_t)st + base + j0 + j, leafThr)) mask |= 1u << (j0 + j);
+        }
+        while (mask) {
+          const int j = __ffs(mask) - 1;
+          mask &= mask - 1;
+          Rec<double, D> r;
+          load_rec(recs, (int64_t)st + base + j, r);
+          const double dist = dist2_seq(q, r);
+          if (within(dist, radLimit) && heap.accepts(dist, r.p.idx) && (a.allowSelf || dist_key(dist) > kEps)) {
+            heap.insert(dist, r.p.idx);
+            changed = true;
+          }
+        }
+      }
+      if (changed) {
+        leafThr = flt.threshold(heap.head(), maxRadius2);
+        pruneThr = prune_threshold();
+      }
+      // pop the next far child that can still hold a better neighbour
+      bool more = false;
+      const unsigned long long popLimit = dist_limit(heap.head());
+      while (sp > 0) {
+        --sp;
+        const uint4 e = stk.entry[sp];
+        if (__uint_as_float(e.y & ~255u) > pruneThr) continue;
+        const int cd = (int)(e.x >> 27);
+        double v[2 * F64Stack<D, STACK>::kPairs];
+#pragma unroll
+        for (int p = 0; p < F64Stack<D, STACK>::kPairs; ++p) {
+          const double2 x = stk.frame[e.y & 255u][p];
+          v[2 * p] = x.x;
+          v[2 * p + 1] = x.y;
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) off2[d] = v[1 + d];
+        const double newOff = Ar<double>::sub(query[cd], __hiloint2double((int)e.w, (int)e.z));
+        const double new2 = Ar<double>::mul(newOff, newOff);
+        const double rdFar = Ar<double>::add(v[0], Ar<double>::add(-pick(off2, cd), new2));
+        if (within(rdFar, radLimit) && within(EXACT ? rdFar : Ar<double>::mul(rdFar, maxError2), popLimit)) {
+          rd = rdFar;
+          rdDown = __double2float_rd(rd);
+#pragma unroll
+          for (int d = 0; d < D; ++d) off2[d] = d == cd ? new2 : off2[d];
+          node = e.x & kMaxNodeIndex;
+          more = true;
+          break;
+        }
+      }
+      if (!more) break;
+    }
+    if (!mayFall || heap.count(k) == k) break;
+    mayFall = false;
+    maxRadius2 = a.maxRadius2;
+    heap.init(k);
+    if (a.fallbacks) atomicAdd(a.fallbacks, 1);
+  }
+  const int f = heap.store(k, a.outIdx + task.outBase, static_cast<double*>(a.outD2) + task.outBase);
+  if (a.found) a.found[task.qi] = f;
   touchedOut += touched;
 }
 
@@ -809,8 +1074,13 @@ __device__ __forceinline__ void knn_kdtree_body(const KnnLaunch& a) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   uint32_t touched = 0;
   if (t < a.nq && (!a.nqDevice || t < (int64_t)*a.nqDevice)) {
-    LocalStack<T, D, STACK> stk;
-    knn_query<T, D, K, EXACT>(a, t, stk, STACK, touched);
+    if constexpr (sizeof(T) == 8) {
+      F64Stack<D, STACK> stk;
+      knn_query_f64<D, K, EXACT, STACK>(a, t, stk, touched);
+    } else {
+      LocalStack<T, D, STACK> stk;
+      knn_query<T, D, K, EXACT>(a, t, stk, STACK, touched);
+    }
   }
   add_touched(a, touched);
 }
@@ -864,7 +1134,7 @@ constexpr size_t deep_stack_bytes(int cap) {
 template <typename T, int D, int K, int STACK, bool EXACT>
 void launch_kdtree_as(int grid, int block, cudaStream_t stream, const KnnLaunch& L) {
   if constexpr (sizeof(T) == 8 && K >= 16)
-    k_knn_kdtree_lean<T, D, K, STACK, EXACT><<<grid, block, 0, stream>>>(L);
+    k_knn_kdtree_lean<T, D, K, STACK, EXACT><<<grid, block, SearchHeap<T, K>::bytes(block), stream>>>(L);
   else
     k_knn_kdtree<T, D, K, STACK, EXACT><<<grid, block, 0, stream>>>(L);
 }
@@ -879,10 +1149,11 @@ void launch_kdtree(int grid, int block, cudaStream_t stream, const KnnLaunch& L)
 
 template <typename T, int D, int K>
 void launch_kdtree_deep(int grid, cudaStream_t stream, const KnnLaunch& L) {
+  constexpr size_t smem = SearchHeap<T, K>::bytes(128);
   if (L.maxError2 == 1.0)
-    k_knn_kdtree_deep<T, D, K, true><<<grid, 128, 0, stream>>>(L);
+    k_knn_kdtree_deep<T, D, K, true><<<grid, 128, smem, stream>>>(L);
   else
-    k_knn_kdtree_deep<T, D, K, false><<<grid, 128, 0, stream>>>(L);
+    k_knn_kdtree_deep<T, D, K, false><<<grid, 128, smem, stream>>>(L);
 }
 
 // Warp-packet traversal for exact search (epsilon = 0).
