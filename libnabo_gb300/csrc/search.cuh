@@ -407,6 +407,7 @@ struct KnnLaunch {
   const int* tallGate;
   int tallGateLimit;
   int32_t* deepFail;
+  int lanes;  // queries per warp, a power of 2 (see spread_lanes): its first lanes search, the others idle
 };
 
 // Leaf scan shared by the kernels: the bucket's records are read in chunks
@@ -1071,9 +1072,10 @@ __device__ __forceinline__ void add_touched(const KnnLaunch& a, uint32_t touched
 template <typename T, int D, int K, int STACK, bool EXACT>
 __device__ __forceinline__ void knn_kdtree_body(const KnnLaunch& a) {
   if (a.tallGate && *a.tallGate > a.tallGateLimit) return;  // the deep kernel searches (uniform)
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int64_t t = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * a.lanes + lane;
   uint32_t touched = 0;
-  if (t < a.nq && (!a.nqDevice || t < (int64_t)*a.nqDevice)) {
+  if (lane < a.lanes && t < a.nq && (!a.nqDevice || t < (int64_t)*a.nqDevice)) {
     if constexpr (sizeof(T) == 8) {
       F64Stack<D, STACK> stk;
       knn_query_f64<D, K, EXACT, STACK>(a, t, stk, touched);

@@ -138,6 +138,23 @@ int launch_wide_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
   return k_unsupported();
 }
 
+// Queries per warp of the one-thread-per-query search. A warp takes as long as
+// its lanes' paths together where they diverge, so a search too small to fill
+// the GPU runs fewer queries in each of more warps: the fewest lanes (a power
+// of 2) that keep at most 16 warps per SM. Search us by queries per warp
+// (32, 16, 8, 4, 2, 1), 3-D lidar map of 1.15 M points, k = 10: 256 queries
+// 167, 137, 117, 99, 84, 72; 4096: 192, 153, 126, 113, 94, 102; 16384: 182,
+// 162, 153, 147, 188, 225; uniform clouds: 10 k queries 51, 46, 41, 42, 49,
+// 60; 30 k: 99, 93, 105, 136, ...; 83 k: 116, 138, 175, ...: past 16 warps
+// per SM the extra warps only repeat instructions.
+inline int spread_lanes(int64_t nq) {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int lanes = 1;
+  while (lanes < 32 && nq > (int64_t)lanes * 16 * sms) lanes *= 2;
+  return lanes;
+}
+
 template <typename T, int D>
 KnnLaunch make_launch(const DeviceCloud& c, const KnnArgs& a, const int32_t* order) {
   KnnLaunch L{};  // every field not set below is zero / null
@@ -180,6 +197,7 @@ KnnLaunch make_launch(const DeviceCloud& c, const KnnArgs& a, const int32_t* ord
   L.tallGate = nullptr;
   L.tallGateLimit = 0;
   L.deepFail = nullptr;
+  L.lanes = 32;
   return L;
 }
 
@@ -197,7 +215,9 @@ int launch_search(const DeviceCloud& c, const KnnArgs& a, const int32_t* order, 
   const int K = round_k(a.k);
   if (K < 0 && a.k > kMaxWideK) return k_unsupported();
   KnnLaunch L = make_launch<T, D>(c, a, order);
-  const int grid = ceil_div(a.nq, 128);
+  L.lanes = spread_lanes(a.nq);
+  const int grid = ceil_div(a.nq, 4 * L.lanes);
+  const int packetGrid = ceil_div(a.nq, 128);
   const bool small = c.height <= kStackSmall;
   // Default: the reference visit order (it is also the faster one on the
   // measured workloads); the warp packet is opt-in for exact searches with
@@ -221,14 +241,14 @@ int launch_search(const DeviceCloud& c, const KnnArgs& a, const int32_t* order, 
   case KK:                                                                         \
     if (packet) {                                                                  \
       if (small)                                                                   \
-        k_knn_kdtree_packet<T, D, KK, kStackSmall><<<grid, 128, 0, stream>>>(L);   \
+        k_knn_kdtree_packet<T, D, KK, kStackSmall><<<packetGrid, 128, 0, stream>>>(L);   \
       else                                                                         \
-        k_knn_kdtree_packet<T, D, KK, kStackLarge><<<grid, 128, 0, stream>>>(L);   \
+        k_knn_kdtree_packet<T, D, KK, kStackLarge><<<packetGrid, 128, 0, stream>>>(L);   \
     } else {                                                                       \
       if (small)                                                                   \
-        launch_kdtree<T, D, KK, kStackSmall>(grid, 128, stream, L);                \
+        launch_kdtree<T, D, KK, kStackSmall>(grid, 128, stream, L);                 \
       else                                                                         \
-        launch_kdtree<T, D, KK, kStackLarge>(grid, 128, stream, L);                \
+        launch_kdtree<T, D, KK, kStackLarge>(grid, 128, stream, L);                 \
     }                                                                              \
     break;
     switch (K) { NABO_K_LIST(NABO_LAUNCH) }
@@ -424,6 +444,7 @@ int search_batch(const BatchArgs& b, int64_t begin, int64_t end, cudaStream_t st
   int rc = kOk;
   KnnLaunch L;
   std::memset(&L, 0, sizeof(L));
+  L.lanes = 32;
   L.nodes = b.nodes;
   L.recs = b.recs;
   L.query = b.query;
@@ -503,7 +524,8 @@ int search_batch(const BatchArgs& b, int64_t begin, int64_t end, cudaStream_t st
       G.runEnd = r1;
       G.nq = cp->runPrefix[(size_t)r1] - cp->runPrefix[(size_t)r0];
       G.k = cp->K[(size_t)gi];
-      const int g = ceil_div(G.nq, b.blockSize);
+      G.lanes = spread_lanes(G.nq);
+      const int g = ceil_div(G.nq, b.blockSize / 32 * G.lanes);
       cudaStream_t gs = stream;
       if (fork && gi != cp->groups - 1) {
         const int a = next++ & 1;
