@@ -79,6 +79,31 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t stream) {
 
 cudaError_t scratch_free(void* p, cudaStream_t stream) { return cudaFreeAsync(p, stream); }
 
+cudaError_t object_alloc(void** p, size_t bytes, cudaStream_t stream) {
+  cudaMemPool_t pool;
+  const cudaError_t e = library_pool(&pool);
+  return e == cudaSuccess ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : e;
+}
+
+cudaError_t object_free(void* const* p, int count) {
+  cudaMemPool_t pool;
+  cudaError_t e = cudaDeviceSynchronize();
+  const cudaError_t pe = library_pool(&pool);
+  for (int i = 0; i < count; ++i) {
+    const cudaError_t fe = p[i] ? cudaFreeAsync(p[i], cudaStreamPerThread) : cudaSuccess;
+    if (e == cudaSuccess) e = fe;
+  }
+  if (pe != cudaSuccess) return pe;
+  uint64_t reserved = 0, used = 0;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      reserved > used + kPoolKeep) {
+    cudaStreamSynchronize(cudaStreamPerThread);
+    cudaMemPoolTrimTo(pool, (size_t)used + kPoolKeep);
+  }
+  return e;
+}
+
 int cuda_error(cudaError_t e, const char* what) {
   g_lastCudaError = e;
   g_lastError = std::string("CUDA error in ") + what + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
@@ -310,8 +335,8 @@ uint32_t storage_bit_count(uint32_t v) {
 // Float copies of a double kd-tree's records for the search's pre-filter.
 template <int D>
 int narrow_cloud_d(DeviceCloud& c, cudaStream_t st) {
-  NABO_CUDA_TRY(cudaMalloc(&c.recs32, (size_t)c.n * sizeof(Rec<float, D>)));
-  NABO_CUDA_TRY(cudaMalloc((void**)&c.coordMax, sizeof(float)));
+  NABO_CUDA_TRY(object_alloc(&c.recs32, (size_t)c.n * sizeof(Rec<float, D>), st));
+  NABO_CUDA_TRY(object_alloc((void**)&c.coordMax, sizeof(float), st));
   return narrow_records<D>(c.recs, c.n, c.dim, c.recs32, c.coordMax, st);
 }
 
@@ -374,10 +399,8 @@ void free_stage(nabo_cuda_search* s) {
 }
 
 void free_cloud(DeviceCloud& c) {
-  if (c.recs) cudaFree(c.recs);
-  if (c.nodes) cudaFree(c.nodes);
-  if (c.recs32) cudaFree(c.recs32);
-  if (c.coordMax) cudaFree(c.coordMax);
+  void* const p[] = {c.recs, c.nodes, c.recs32, c.coordMax};
+  object_free(p, 4);
   c.recs = nullptr;
   c.nodes = nullptr;
   c.recs32 = nullptr;
