@@ -11,9 +11,9 @@
 // Phases:
 //   1. pack + bounds: records in cloud order, per-dimension min/max.
 //   2. top levels, all segments of a level at once: the reference's rule in
-//      one cooperative launch down to segments that fit in shared memory
-//      (k_top), the median rule as a stable scatter per level down to 256
-//      points (k_median_*).
+//      one cooperative launch (k_top), the median rule as a stable scatter per
+//      level (k_median_*), down to segments that fit in a block's shared
+//      memory.
 //   3. small segments: a block each (or several at once) splits its points in
 //      shared memory down to leaves (k_mid).
 //   4. numbering: splits and leaves are recorded by position; a count of the
@@ -32,7 +32,6 @@ namespace nabo_gb300 {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kSmallMax = 256;
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ int2 add2(int2 a, int2 b) { return make_int2(a.x + b.x, a.y + b.y); }
@@ -203,56 +202,7 @@ __device__ __forceinline__ void warp_sort_keys(Key (&e)[R], int lane) {
   }
 }
 
-// The lower median (rank count / 2) of the count values node[i].p.c[cd],
-// computed by the warp over the values' order-preserving keys (padding
-// sorts above every finite value's key, so it never holds the rank). Up to
-// 64 values a bitonic sort across the warp (one or two keys per lane) and
-// the key at the rank; above, a bitwise radix select, most significant bit
-// first: each round counts the remaining candidates whose next bit is 0 (one
-// compare per held value, summed across the warp) and keeps the half that
-// holds the rank, 32 rounds for float and 64 for double.
-template <typename T, int D>
-__device__ T warp_median(const Rec<T, D>* node, int count, int cd, int lane) {
-  using Key = typename KeyOf<T>::type;
-  const int want0 = count / 2;
-  if (count <= 32) {
-    Key e[1] = {lane < count ? ordered_key(node[lane].p.c[cd]) : ~Key(0)};
-    warp_sort_keys<1>(e, lane);
-    return ordered_val(__shfl_sync(0xffffffffu, e[0], want0), T(0));
-  }
-  if (count <= 64) {
-    Key e[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) e[r] = lane + 32 * r < count ? ordered_key(node[lane + 32 * r].p.c[cd]) : ~Key(0);
-    warp_sort_keys<2>(e, lane);
-    const Key m = __shfl_sync(0xffffffffu, want0 >= 32 ? e[1] : e[0], want0 & 31);
-    return ordered_val(m, T(0));
-  }
-  constexpr int kPer = kSmallMax / 32;
-  constexpr int kBits = 8 * (int)sizeof(Key);
-  Key k[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int i = lane + 32 * j;
-    // padding sorts above every finite value's key, so it never holds the rank
-    k[j] = i < count ? ordered_key(node[i].p.c[cd]) : ~Key(0);
-  }
-  const int held = (count + 31) / 32;
-  Key prefix = 0;
-  int want = want0;
-  for (int b = kBits - 1; b >= 0; --b) {
-    const Key sel = prefix >> b;
-    int c = 0;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) c += (j < held && (k[j] >> b) == sel) ? 1 : 0;
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (want >= c) {
-      want -= c;
-      prefix |= Key(1) << b;
-    }
-  }
-  return ordered_val(prefix, T(0));
-}
+constexpr int kMedianSamples = 31;
 
 }  // namespace
 }  // namespace nabo_gb300
@@ -308,12 +258,11 @@ __device__ __forceinline__ int arg_max_extent(const T* lo, const T* hi, int dim)
 // Median-split trees (split rule 1): the cut is just above the median of the
 // segment's coordinates along the cut dimension (sampled at kMedianSamples
 // evenly spaced positions at the level-synchronous levels, where the
-// segment's points are in no particular order; exact in k_small). Just above
+// segment's points are in no particular order; exact below kHeld points, in
+// k_mid). Just above
 // (the next representable value): points equal to the median go left and
 // hardly any point lies on the cut, so the build's second partition pass,
 // which only segments with points on their cut run, is skipped.
-constexpr int kMedianSamples = 31;
-
 template <typename T>
 __device__ T sampled_median(const T* __restrict__ val, int start, int count) {
   T smp[kMedianSamples];
@@ -364,7 +313,7 @@ __global__ void k_scan_block_sums(int2* sums, int nb, int2* total, const LevelSt
 template <typename T, int D>
 __device__ void emit_split(const SegLevel<T>& L, const SegLevel<T>& next, int s, int leftCount, int cd, T cut,
                            const SegList<T>& small, const TreeMarks<T>& marks, int* counters, int dim, int bucket,
-                           int segCap, int smallCap, int level) {
+                           int smallMax, int segCap, int smallCap, int level) {
   const int count = L.count[s];
   const int start = L.start[s];
   const int turns = L.turns[s];
@@ -382,7 +331,7 @@ __device__ void emit_split(const SegLevel<T>& L, const SegLevel<T>& next, int s,
     if (ccount <= bucket) {
       mark_leaf(marks, cst, cturns);
       atomicMax(counters + kHeight, level + 1);
-    } else if (ccount > kSmallMax) {
+    } else if (ccount > smallMax) {
       const int id = atomicAdd(counters + kNextSegs, 1);
       if (id >= segCap) {
         atomicOr(counters + kFlags, 1);
@@ -580,8 +529,8 @@ __global__ void k_median_sums(MedianBufs<T, D> B, int64_t nPad, SegLevel<T> L, i
 // L.lt keeps the chosen flag's global rank at the segment's first position.
 template <typename T, int D>
 __global__ void k_median_split(SegLevel<T> L, SegLevel<T> next, const LevelState* st, SegList<T> small,
-                               TreeMarks<T> marks, int* counters, int dim, int bucket, int segCap, int smallCap,
-                               const int2* __restrict__ blockPrefix, const int2* __restrict__ segFirst,
+                               TreeMarks<T> marks, int* counters, int dim, int bucket, int smallMax, int segCap,
+                               int smallCap, const int2* __restrict__ blockPrefix, const int2* __restrict__ segFirst,
                                const int2* __restrict__ segLast, int perBlock) {
   pdl_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -612,8 +561,8 @@ __global__ void k_median_split(SegLevel<T> L, SegLevel<T> next, const LevelState
   }
   leftCount = leftCount < 1 ? 1 : (leftCount > count - 1 ? count - 1 : leftCount);
   L.mode[s] = mode;
-  emit_split<T, D>(L, next, s, leftCount, L.cutDim[s], cut, small, marks, counters, dim, bucket, segCap, smallCap,
-                   st->level);
+  emit_split<T, D>(L, next, s, leftCount, L.cutDim[s], cut, small, marks, counters, dim, bucket, smallMax, segCap,
+                   smallCap, st->level);
 }
 
 // Moves every record of a large segment to its child's range: a record with
@@ -1140,15 +1089,14 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   const int rangeBlocks = std::max(1, std::min(ceil_div(std::max<int64_t>(n, 1), kBlock), 8 * sms));
   const int64_t rangeChunk = (int64_t)ceil_div(ceil_div(std::max<int64_t>(n, 1), rangeBlocks), kBlock) * kBlock;
 
-  // Small segments: the reference's rule hands over what fits in a block's
-  // shared memory, the median rule its 256-point segments, several to a block.
-  const int midCap = median ? std::min(Mid::kMax, 2048) : Mid::kMax;
-  const int smallMax = median ? kSmallMax : Mid::kMax;
-  const int midThreads = median ? 256 : Mid::kThreads;
-  const size_t midSmem = Mid::smem(midCap, bucket);
+  // Small segments: what a block of k_mid holds in shared memory. (Median
+  // rule, 512 clouds of 21 M points, built and searched: handed over at 256
+  // points 18.8 ms, 1024 18.3, 2048 18.1, 4096 17.9.)
+  const int smallMax = Mid::kMax;
+  const size_t midSmem = Mid::smem(smallMax, bucket);
   NABO_CUDA_TRY(cudaFuncSetAttribute(k_mid<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)midSmem));
   int midOcc = 0;
-  NABO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&midOcc, k_mid<T, D>, midThreads, midSmem));
+  NABO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&midOcc, k_mid<T, D>, Mid::kThreads, midSmem));
 
   // k_top: one block per SM, each with its share of the positions
   const bool top = !median && n > smallMax;
@@ -1303,7 +1251,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
                                segFirst, segLast, st));
       NABO_CUDA_TRY(launch_pdl(k_scan_block_sums, 1, kBlock, 0, stream, blockSums, mBlocks, passTotal, st));
       NABO_CUDA_TRY(launch_pdl(k_median_split<T, D>, sg, 128, 0, stream, cur, nxt, st, small, marks, counters, dim,
-                               bucket, (int)segCap, (int)smallCap, (const int2*)blockSums, (const int2*)segFirst,
+                               bucket, smallMax, (int)segCap, (int)smallCap, (const int2*)blockSums, (const int2*)segFirst,
                                (const int2*)segLast, mTiles * kTile));
       NABO_CUDA_TRY(launch_pdl(median_scatter<T, D>(), mBlocks, kBlock, 0, stream, mb, recs, nPad, cur, nxt, mTiles,
                                (const int2*)blockSums, st));
@@ -1323,12 +1271,12 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   ma.nonFinite = nonFinite;
   ma.dim = dim;
   ma.bucket = bucket;
-  ma.cap = midCap;
-  ma.claim = std::max(1, std::min(32, median ? midCap / smallMax : 16));
+  ma.cap = smallMax;
+  ma.claim = 16;
   ma.maxLevels = maxLevels;
   ma.splitRule = splitRule;
   const int midGrid = (int)std::min<int64_t>(smallCap, (int64_t)std::max(midOcc, 1) * sms);
-  k_mid<T, D><<<midGrid, midThreads, midSmem, stream>>>(ma);
+  k_mid<T, D><<<midGrid, Mid::kThreads, midSmem, stream>>>(ma);
   NABO_CUDA_TRY(cudaGetLastError());
 
   k_leaf_ranks<<<rankBlocks, kRankBlock, 0, stream>>>(marks.leafBits, words, rank, rankSums);

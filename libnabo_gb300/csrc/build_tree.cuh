@@ -611,6 +611,7 @@ struct MidNode {
 template <typename T, int D>
 struct MidShape {
   static constexpr int kThreads = sizeof(Rec<T, D>) <= 32 ? 512 : 256;
+  static constexpr int kBlocks = sizeof(Rec<T, D>) <= 16 ? 2 : 1;  // per SM at least
   // largest segment of the reference's rule
   static constexpr int kMax = sizeof(Rec<T, D>) <= 16   ? 4096
                               : sizeof(Rec<T, D>) <= 48 ? 2048
@@ -673,6 +674,116 @@ __device__ __forceinline__ float warp_max_val(float v) { return ordered_val(__re
 __device__ __forceinline__ double warp_min_val(double v) { return warp_min(v); }
 __device__ __forceinline__ double warp_max_val(double v) { return warp_max(v); }
 
+__device__ __forceinline__ uint32_t warp_or(uint32_t v) { return __reduce_or_sync(kFull, v); }
+__device__ __forceinline__ uint32_t warp_and(uint32_t v) { return __reduce_and_sync(kFull, v); }
+__device__ __forceinline__ unsigned long long warp_or(unsigned long long v) {
+  return (unsigned long long)warp_or((uint32_t)(v >> 32)) << 32 | warp_or((uint32_t)v);
+}
+__device__ __forceinline__ unsigned long long warp_and(unsigned long long v) {
+  return (unsigned long long)warp_and((uint32_t)(v >> 32)) << 32 | warp_and((uint32_t)v);
+}
+
+// The middle one of 31 values sampled evenly, as the median rule's top levels
+// take it.
+template <typename T, int D>
+__device__ __forceinline__ T warp_sampled_median(const Rec<T, D>* node, int count, int cd, int lane) {
+  using Key = typename KeyOf<T>::type;
+  Key e[1] = {lane < kMedianSamples ? ordered_key(node[(int)((int64_t)(2 * lane + 1) * count / (2 * kMedianSamples))].p.c[cd])
+                                    : ~Key(0)};
+  warp_sort_keys<1>(e, lane);
+  return ordered_val(__shfl_sync(kFull, e[0], kMedianSamples / 2), T(0));
+}
+
+// The lower median (rank count / 2) of up to kHeld values, by a warp holding
+// every 32nd of them in each lane: bit by bit below the bits that all keys
+// share, until one candidate is left (about 11 rounds instead of a bit each).
+constexpr int kHeld = 256;
+template <typename T, int D>
+__device__ __forceinline__ T warp_median(const Rec<T, D>* node, int count, int cd, int lane) {
+  using Key = typename KeyOf<T>::type;
+  constexpr int kPer = kHeld / 32;
+  const int held = (count + 31) >> 5;
+  Key k[kPer];
+  Key any = 0, all = ~Key(0);
+  unsigned alive = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    k[j] = 0;
+    if (j < held && lane + 32 * j < count) {
+      k[j] = ordered_key(node[lane + 32 * j].p.c[cd]);
+      any |= k[j];
+      all &= k[j];
+      alive |= 1u << j;
+    }
+  }
+  any = warp_or(any);
+  const Key diff = any & ~warp_and(all);  // bits in which some keys differ
+  int left = count, want = count / 2;
+  for (int b = 8 * (int)sizeof(Key) - 1; b >= 0 && left > 1; --b) {
+    if (!((diff >> b) & 1)) continue;
+    unsigned zeros = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) zeros |= ((k[j] >> b) & 1) ? 0u : 1u << j;
+    zeros &= alive;
+    const int c = __reduce_add_sync(kFull, __popc(zeros));
+    if (want < c) {
+      alive = zeros;
+      left = c;
+    } else {
+      want -= c;
+      alive &= ~zeros;
+      left -= c;
+    }
+  }
+  Key m = k[0];
+#pragma unroll
+  for (int j = 1; j < kPer; ++j)
+    if ((alive & ((1u << j) - 1u)) == 0u) m = k[j];
+  const int src = __ffs(__ballot_sync(kFull, alive != 0u)) - 1;
+  return ordered_val(__shfl_sync(kFull, m, src), T(0));
+}
+
+// Splits a node, by a warp, at `ideal` (the median rule: just above it, so
+// that points equal to it go left and hardly any lies on the cut) and
+// partitions by v < cut, or v <= cut below the minimum. Returns the mode.
+// `sampled`: a sampled median with nothing above it divides the points on it
+// by position.
+template <typename T, int D>
+__device__ __forceinline__ int split_node(Rec<T, D>* pts, int count, int cd, T ideal, bool sampled, uint16_t* tab,
+                                          int lane, T* cutOut, int* ltOut, int* eqOut) {
+  T mn = std::numeric_limits<T>::max(), mx = std::numeric_limits<T>::lowest();
+  int lt = 0, eq = 0;
+#pragma unroll 4
+  for (int j = lane; j < count; j += 32) {
+    const T v = pts[j].p.c[cd];
+    mn = v < mn ? v : mn;
+    mx = v > mx ? v : mx;
+    lt += v < ideal ? 1 : 0;
+    eq += v == ideal ? 1 : 0;
+  }
+  mn = warp_min_val(mn);
+  mx = warp_max_val(mx);
+  lt = __reduce_add_sync(kFull, lt);
+  eq = __reduce_add_sync(kFull, eq);
+  int mode = kInside;
+  T cut = ideal;
+  if (ideal < mn || ideal > mx) {  // the points on a clamped cut
+    mode = ideal < mn ? kBelowMin : kAboveMax;
+    cut = ideal < mn ? mn : mx;
+    eq = 0;
+    for (int j = lane; j < count; j += 32) eq += pts[j].p.c[cd] == cut ? 1 : 0;
+    eq = __reduce_add_sync(kFull, eq);
+    lt = mode == kBelowMin ? 0 : lt - eq;  // above the maximum, lt counted every point
+    if (sampled) mode = kInside;
+  }
+  *cutOut = cut;
+  *ltOut = lt;
+  *eqOut = eq;
+  const bool lessEq = mode == kBelowMin;
+  warp_partition<T, D>(pts, count, lessEq ? eq : lt, cd, cut, lessEq, tab, lane);
+  return mode;
+}
+
 // A record from another lane.
 template <typename T, int D>
 __device__ __forceinline__ Rec<T, D> shfl_rec(const Rec<T, D>& r, int src) {
@@ -688,7 +799,7 @@ __device__ __forceinline__ Rec<T, D> shfl_rec(const Rec<T, D>& r, int src) {
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(MidShape<T, D>::kThreads) k_mid(const MidArgs<T, D> a) {
+__global__ void __launch_bounds__(MidShape<T, D>::kThreads, MidShape<T, D>::kBlocks) k_mid(const MidArgs<T, D> a) {
   using Node = MidNode<T, D>;
   extern __shared__ __align__(16) unsigned char midSmem[];
   __shared__ int listCount[2], jobCount, claimAt, take, total;
@@ -805,35 +916,12 @@ __global__ void __launch_bounds__(MidShape<T, D>::kThreads) k_mid(const MidArgs<
           }
           T ideal;
           const int cd = widest_dim<T, D>(N.lo, N.hi, a.dim, &ideal);
-          if (a.splitRule == 1) ideal = next_up(warp_median(node, count, cd, lane));
-          T mn = std::numeric_limits<T>::max(), mx = std::numeric_limits<T>::lowest();
-          int lt = 0, eq = 0;
-#pragma unroll 4
-          for (int j = lane; j < count; j += 32) {
-            const T v = node[j].p.c[cd];
-            mn = v < mn ? v : mn;
-            mx = v > mx ? v : mx;
-            lt += v < ideal ? 1 : 0;
-            eq += v == ideal ? 1 : 0;
-          }
-          mn = warp_min_val(mn);
-          mx = warp_max_val(mx);
-          lt = __reduce_add_sync(kFull, lt);
-          eq = __reduce_add_sync(kFull, eq);
-          int mode = kInside;
-          T cut = ideal;
-          if (ideal < mn || ideal > mx) {  // a clamped cut: count the points on it
-            mode = ideal < mn ? kBelowMin : kAboveMax;
-            cut = ideal < mn ? mn : mx;
-            eq = 0;
-            for (int j = lane; j < count; j += 32) eq += node[j].p.c[cd] == cut ? 1 : 0;
-            eq = __reduce_add_sync(kFull, eq);
-            lt = mode == kBelowMin ? 0 : lt - eq;  // above the maximum, lt counted every point
-          }
-          if (mode == kBelowMin)
-            warp_partition<T, D>(node, count, eq, cd, cut, true, tab + N.st, lane);
-          else
-            warp_partition<T, D>(node, count, lt, cd, cut, false, tab + N.st, lane);
+          int mode, lt, eq;
+          T cut;
+          const bool median = a.splitRule == 1, sampled = median && count > kHeld;
+          if (median)
+            ideal = next_up(sampled ? warp_sampled_median(node, count, cd, lane) : warp_median(node, count, cd, lane));
+          mode = split_node<T, D>(node, count, cd, ideal, sampled, tab + N.st, lane, &cut, &lt, &eq);
           if (mode == kInside && eq > 0)
             warp_partition<T, D>(node + lt, count - lt, eq, cd, cut, true, tab + N.st + lt, lane);
           const int l = left_count(mode, count, lt, eq);
