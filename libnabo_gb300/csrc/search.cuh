@@ -1266,7 +1266,8 @@ __global__ void __launch_bounds__(128) k_knn_kdtree_packet(KnnLaunch a) {
 }
 
 // Brute force (nabo/brute_force_cpu.cpp:63-103): every query against every
-// point. The points are staged through shared memory in tiles of 24 KB; a
+// point. Doubles, and float clouds of fewer than 512 points or of a range that
+// k_bf_tc does not take, run here. The points are staged through shared memory in tiles of 24 KB; a
 // thread owns QT queries (blockDim.x apart) and their top-k, so each record
 // read from shared memory (a broadcast: every lane reads the same one) feeds
 // QT distances. The distance is the reference's separately rounded

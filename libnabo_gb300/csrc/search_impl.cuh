@@ -2,11 +2,13 @@
 // Included by one translation unit per (T, D) so they compile in parallel.
 #pragma once
 
+#include "bruteforce_tc.cuh"
 #include "internal.cuh"
 #include "search.cuh"
 #include "search_wide.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 
@@ -346,6 +348,89 @@ int launch_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
   return kOk;
 }
 
+// Centre and scale of the tensor-core filter's coordinates; false when the
+// cloud's range does not suit it.
+inline bool tc_scale(const DeviceCloud& c, TcScale* s) {
+  double half[kMaxDim], widest = 0.0;
+  for (int d = 0; d < kMaxDim; ++d) {
+    s->centre[d] = 0.0f;
+    if (d >= c.dim) continue;
+    if (!(std::fabs(c.lo[d]) < 1e15 && std::fabs(c.hi[d]) < 1e15)) return false;
+    s->centre[d] = (float)(0.5 * (c.lo[d] + c.hi[d]));
+    half[d] = std::max(c.hi[d] - (double)s->centre[d], (double)s->centre[d] - c.lo[d]);
+    widest = std::max(widest, half[d]);
+  }
+  if (!(widest > 1e-15)) return false;
+  int e = 0;
+  std::frexp(widest, &e);  // widest <= 2^e
+  s->scale = (float)std::ldexp(1.0, -e);
+  s->scale2 = s->scale * s->scale;
+  double p = 0.0;
+  for (int d = 0; d < c.dim; ++d) p += half[d] * half[d] * s->scale2;
+  s->pointMax = (float)std::max(0.25, p * (1.0 + 1e-5));
+  return true;
+}
+
+// Block rows (parts of the points) of a search of qBlocks query blocks when
+// `slots` blocks run at once: fewest waves per row (the last, partly empty one
+// counted as 0.4 of one more), each further row costing 4 + k percent (at
+// most 25) for lists that start empty. (100 k x 100 k points, 1, 2, 3 and 4 rows, ms: k = 5
+// 1.62, 1.55, 1.61, 1.70; k = 16 2.47, 2.73, 2.95, 3.17; 40 k queries in 8-D:
+// 0.56, 0.57, 0.52, 0.55.)
+inline int64_t tc_rows(int64_t qBlocks, int64_t slots, int64_t most, int k) {
+  const double rowCost = std::min(0.25, 0.04 + 0.01 * k);
+  int64_t best = 1;
+  double least = 0.0;
+  for (int64_t r = 1; r <= std::max<int64_t>(most, 1); ++r) {
+    const double waves = (double)(qBlocks * r) / (double)slots;
+    const double cost = (waves <= 1.0 ? 1.0 : waves + 0.4) / (double)r * (1.0 + rowCost * (double)(r - 1));
+    if (r == 1 || cost < least) {
+      least = cost;
+      best = r;
+    }
+  }
+  return best;
+}
+
+template <int D, int K>
+int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, cudaStream_t stream) {
+  using S = TcSmem<D, K>;
+  const int qBlocks = ceil_div(L.nq, kTcQueries);
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t stages = (L.n + S::kStagePoints - 1) / S::kStagePoints;
+  const int perSm = std::min(TcTile<K>::kBlocksPerSm, 228 * 1024 / (S::kRequest + 1024));
+  int64_t rows = tc_rows(qBlocks, (int64_t)perSm * sms, std::min<int64_t>(stages / kTcSeedStride, 64), L.k);
+  const int64_t chunk = (stages + rows - 1) / rows * S::kStagePoints;
+  rows = (L.n + chunk - 1) / chunk;
+  const int64_t padded = stages * S::kStagePoints;
+  const int64_t stride = rows > 1 ? L.nq * (int64_t)L.k : 0;
+  const size_t operandBytes = TcShape<D>::operandBytes(1) * (size_t)padded;
+  const size_t idxBytes = ((size_t)(rows * stride) * sizeof(int32_t) + 255) / 256 * 256;
+  unsigned char* block = nullptr;  // operand | partial indices | partial distances
+  NABO_CUDA_TRY(scratch_alloc((void**)&block, operandBytes + 2 * idxBytes, stream));
+  k_bf_tc_points<D><<<ceil_div(padded, 256), 256, 0, stream>>>(static_cast<const Rec<float, D>*>(L.recs), L.n, padded,
+                                                               L.dim, s, block);
+  constexpr int smem = S::kRequest;
+  cudaError_t e = cudaFuncSetAttribute(k_bf_tc<D, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  KnnLaunch P = L;
+  if (rows > 1) {
+    P.outIdx = reinterpret_cast<int32_t*>(block + operandBytes);
+    P.outD2 = block + operandBytes + idxBytes;
+    P.found = nullptr;
+  }
+  if (e == cudaSuccess) {
+    k_bf_tc<D, K><<<dim3(qBlocks, (unsigned)rows), kTcThreads, smem, stream>>>(P, block, s, chunk, stride);
+    if (rows > 1)
+      k_bf_merge<float, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(P.outIdx, static_cast<const float*>(P.outD2),
+                                                                    (int)rows, stride, L.nq, L.k, L.outIdx,
+                                                                    static_cast<float*>(L.outD2), L.found);
+    e = cudaGetLastError();
+  }
+  scratch_free(block, stream);
+  return e == cudaSuccess ? kOk : cuda_error(e, "tensor-core brute force");
+}
+
 template <typename T, int D>
 int knn_bruteforce(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream) {
   if (a.nq == 0) return kOk;
@@ -355,11 +440,27 @@ int knn_bruteforce(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream) 
   if (a.evStart) cudaEventRecord(a.evStart, stream);
   int rc = kOk;
   if (K < 0) rc = launch_wide_bruteforce<T, D>(L, stream);
+  bool done = K < 0;
+  if constexpr (sizeof(T) == 4) {
+    TcScale s;
+    // (us, without / with the tensor cores: 64 points, 100 k queries 35 / 59;
+    // 256 points 90 / 93; 500 points, 5 k queries 59 / 48; 100 k points, one
+    // query 176 / 71)
+    if (!done && c.n >= 512 && tc_scale(c, &s)) {
+#define NABO_LAUNCH(KK)                                   \
+  case KK:                                                \
+    rc = launch_bruteforce_tc<D, KK>(L, s, stream);       \
+    break;
+      switch (K) { NABO_K_LIST(NABO_LAUNCH) }
+#undef NABO_LAUNCH
+      done = true;
+    }
+  }
 #define NABO_LAUNCH(KK)                                 \
   case KK:                                              \
     rc = launch_bruteforce<T, D, KK>(L, stream);        \
     break;
-  if (K > 0) switch (K) { NABO_K_LIST(NABO_LAUNCH) }
+  if (!done) switch (K) { NABO_K_LIST(NABO_LAUNCH) }
 #undef NABO_LAUNCH
   if (a.evStop) cudaEventRecord(a.evStop, stream);
   if (rc != kOk) return rc;
