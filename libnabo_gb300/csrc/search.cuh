@@ -18,8 +18,8 @@
 // result independent of visit order (the reference's
 // IndexHeapBruteForceVector keeps the first visited, nabo/index_heap.h:
 // 322-334). Insertion is branch-free: with g[j] = (slot j > new entry),
-// which is true for a prefix of the slots, slot j takes slot j+1 while
-// g[j+1], the new entry where the prefix ends, and keeps its value after.
+// which is true for a prefix of the slots, slot j takes the new entry while
+// g[j], then slot j+1 while g[j+1], and keeps its value after (move_if).
 #pragma once
 
 #include <type_traits>
@@ -27,6 +27,35 @@
 #include "common.cuh"
 
 namespace nabo_gb300 {
+
+// dst = src where p, as a predicated multiply-add by a one the compiler cannot
+// see through (an integer src * 1 + 0, on the FMA pipe). The searches are bound
+// by the ALU pipe, which executes selects and compares; written as selects, an
+// insertion into a sorted register list took two thirds of its ALU slots for
+// moving entries. (Search kernel, selects -> predicated moves, which the
+// compiler turns back into selects for the most part -> these: lidar 1.15 M
+// points and queries, k = 10 1053 -> 940 -> 877 us; uniform 1 M 850 -> 768 ->
+// 735; lidar 500 k, k = 16 695 -> 620 -> 580; the 512-cloud batch 18.3 -> 16.7
+// -> 15.95 ms. The same for the traversal's coordinate picks was slower, 877
+// -> 940: they wait on the multiplies' latency.)
+static __constant__ uint32_t c_one = 1u;
+__device__ __forceinline__ void move_if(bool p, uint32_t& dst, uint32_t src, uint32_t one) {
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p mad.lo.u32 %0, %1, %3, 0;\n\t}"
+      : "+r"(dst)
+      : "r"(src), "r"((int)p), "r"(one));
+}
+__device__ __forceinline__ void move_if(bool p, int& dst, int src, uint32_t one) {
+  uint32_t d = (uint32_t)dst;
+  move_if(p, d, (uint32_t)src, one);
+  dst = (int)d;
+}
+template <typename U>
+__device__ __forceinline__ std::enable_if_t<sizeof(U) == 8> move_if(bool p, U& dst, U src, uint32_t one) {
+  uint32_t l = (uint32_t)dst, h = (uint32_t)(dst >> 32);
+  move_if(p, l, (uint32_t)src, one);
+  move_if(p, h, (uint32_t)(src >> 32), one);
+  dst = (U)h << 32 | l;
+}
 
 // double: the distance's 64-bit pattern and the index in separate arrays.
 // Distances are >= 0, where the pattern orders like the value, so the
@@ -56,16 +85,18 @@ struct TopK {
   // Drops the head and inserts (dist, idx); requires accepts(dist, idx).
   __device__ __forceinline__ void insert(T dist, int idx) {
     const unsigned long long x = bits(dist);
-    bool g[K];
+    const uint32_t one = c_one;
+    bool g = true;  // entry j > (dist, idx)
 #pragma unroll
-    for (int j = 0; j < K; ++j) g[j] = greater(d[j], i[j], x, idx);
-#pragma unroll
-    for (int j = 0; j + 1 < K; ++j) {
-      d[j] = g[j + 1] ? d[j + 1] : (g[j] ? x : d[j]);
-      i[j] = g[j + 1] ? i[j + 1] : (g[j] ? idx : i[j]);
+    for (int j = 0; j < K; ++j) {
+      move_if(g, d[j], x, one);
+      move_if(g, i[j], idx, one);
+      if (j + 1 < K) {
+        g = greater(d[j + 1], i[j + 1], x, idx);
+        move_if(g, d[j], d[j + 1], one);
+        move_if(g, i[j], i[j + 1], one);
+      }
     }
-    d[K - 1] = g[K - 1] ? x : d[K - 1];
-    i[K - 1] = g[K - 1] ? idx : i[K - 1];
   }
   __device__ __forceinline__ int count(int k) const {
     int c = 0;
@@ -222,12 +253,16 @@ struct TopK<float, K> {
   __device__ __forceinline__ void insert(float dist, int idx) { insert_key(make(dist, idx)); }
   // requires x < key[0]
   __device__ __forceinline__ void insert_key(uint64_t x) {
-    bool g[K];
+    const uint32_t one = c_one;
+    bool g = true;  // key[j] > x
 #pragma unroll
-    for (int j = 0; j < K; ++j) g[j] = key[j] > x;
-#pragma unroll
-    for (int j = 0; j + 1 < K; ++j) key[j] = g[j + 1] ? key[j + 1] : (g[j] ? x : key[j]);
-    key[K - 1] = g[K - 1] ? x : key[K - 1];
+    for (int j = 0; j < K; ++j) {
+      move_if(g, key[j], x, one);
+      if (j + 1 < K) {
+        g = key[j + 1] > x;
+        move_if(g, key[j], key[j + 1], one);
+      }
+    }
   }
   __device__ __forceinline__ int count(int k) const {
     int c = 0;
@@ -306,8 +341,9 @@ __device__ __forceinline__ T pick(const T (&v)[D], int c) {
   } else {
     T r = v[0];
 #pragma unroll
-    for (int d = 1; d < D; ++d)
+    for (int d = 1; d < D; ++d) {
       if (c == d) r = v[d];
+    }
     return r;
   }
 }
@@ -496,6 +532,8 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
       const uint64_t thrKey =
           (!want || radKey == 0ull) ? 0ull : (heap.key[0] <= radKey ? heap.key[0] : radKey + 1ull);
       uint64_t kj[kChunk];
+      const float hd = heap.head();
+      const float thrF = want ? (hd < maxRadius2 ? hd : maxRadius2) : __int_as_float(0x7fffffff);
 #pragma unroll
       for (int j = 0; j < kChunk; ++j) {
         kj[j] = ~0ull;
@@ -504,7 +542,7 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
           load_rec(recs, (int64_t)st + base + j, r);
           const float d = dist2_seq(q, r);
           kj[j] = TopK<float, K>::make(d, r.p.idx);
-          mask |= (kj[j] < thrKey && d > minDist) ? (1u << j) : 0u;
+          mask |= (d <= thrF && d > minDist) ? (1u << j) : 0u;
         }
       }
       while (mask) {
@@ -512,8 +550,9 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
         mask &= mask - 1;
         uint64_t v = kj[0];
 #pragma unroll
-        for (int m = 1; m < kChunk; ++m)
+        for (int m = 1; m < kChunk; ++m) {
           if (j == m) v = kj[m];
+        }
         if (v < heap.key[0]) heap.insert_key(v);
       }
     } else {
@@ -651,7 +690,9 @@ __device__ __forceinline__ void stack_push(StackRec<T, D>& e, T rd, const T (&of
   for (int i = 0; i < R::kChunks * 4; ++i) w[i] = 0u;
   put_t(w, 0, rd);
 #pragma unroll
-  for (int d = 0; d < D; ++d) put_t(w, R::kTW * (1 + d), d == cd ? new2 : off2[d]);
+  for (int d = 0; d < D; ++d) {
+    put_t(w, R::kTW * (1 + d), d == cd ? new2 : off2[d]);
+  }
   w[R::kNode] = node;
 #pragma unroll
   for (int c = 0; c < R::kChunks; ++c) {

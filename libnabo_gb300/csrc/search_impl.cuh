@@ -408,7 +408,10 @@ int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, cudaStream_t stre
   const size_t operandBytes = TcShape<D>::operandBytes(1) * (size_t)padded;
   const size_t idxBytes = ((size_t)(rows * stride) * sizeof(int32_t) + 255) / 256 * 256;
   unsigned char* block = nullptr;  // operand | partial indices | partial distances
-  NABO_CUDA_TRY(scratch_alloc((void**)&block, operandBytes + 2 * idxBytes, stream));
+  if (scratch_alloc((void**)&block, operandBytes + 2 * idxBytes, stream) != cudaSuccess) {
+    cudaGetLastError();  // no room for the operand: the kernel that needs none
+    return launch_bruteforce<float, D, K>(L, stream);
+  }
   k_bf_tc_points<D><<<ceil_div(padded, 256), 256, 0, stream>>>(static_cast<const Rec<float, D>*>(L.recs), L.n, padded,
                                                                L.dim, s, block);
   constexpr int smem = S::kRequest;

@@ -56,12 +56,15 @@ struct GroupTopK<float, M, G> {
   __device__ __forceinline__ void insert_key(uint64_t x, int g, unsigned gm) {
     uint64_t prev = __shfl_up_sync(gm, a[M - 1], 1, G);
     if (g == 0) prev = 0ull;
-    bool gt[M];
+    const uint32_t one = c_one;
+    bool gt = a[M - 1] > x;
 #pragma unroll
-    for (int r = 0; r < M; ++r) gt[r] = a[r] > x;
-#pragma unroll
-    for (int r = M - 1; r >= 1; --r) a[r] = gt[r] ? (gt[r - 1] ? a[r - 1] : x) : a[r];
-    a[0] = gt[0] ? (prev > x ? prev : x) : a[0];
+    for (int r = M - 1; r >= 0; --r) {
+      const uint64_t lower = r > 0 ? a[r > 0 ? r - 1 : 0] : prev;
+      move_if(gt, a[r], x, one);
+      gt = lower > x;  // implies a[r] > x
+      move_if(gt, a[r], lower, one);
+    }
     h = __shfl_sync(gm, a[M - 1], G - 1, G);
   }
   __device__ __forceinline__ int count(int k, int g, unsigned gm) const {
@@ -122,17 +125,18 @@ struct GroupTopK<double, M, G> {
       pd = 0ull;
       pi = -1;
     }
-    bool gt[M];
+    const uint32_t one = c_one;
+    bool gt = greater(d[M - 1], i[M - 1], x, idx);
 #pragma unroll
-    for (int r = 0; r < M; ++r) gt[r] = greater(d[r], i[r], x, idx);
-#pragma unroll
-    for (int r = M - 1; r >= 1; --r) {
-      d[r] = gt[r] ? (gt[r - 1] ? d[r - 1] : x) : d[r];
-      i[r] = gt[r] ? (gt[r - 1] ? i[r - 1] : idx) : i[r];
+    for (int r = M - 1; r >= 0; --r) {
+      const unsigned long long ld = r > 0 ? d[r > 0 ? r - 1 : 0] : pd;
+      const int li = r > 0 ? i[r > 0 ? r - 1 : 0] : pi;
+      move_if(gt, d[r], x, one);
+      move_if(gt, i[r], idx, one);
+      gt = greater(ld, li, x, idx);  // implies entry r is greater
+      move_if(gt, d[r], ld, one);
+      move_if(gt, i[r], li, one);
     }
-    const bool gp = greater(pd, pi, x, idx);
-    d[0] = gt[0] ? (gp ? pd : x) : d[0];
-    i[0] = gt[0] ? (gp ? pi : idx) : i[0];
     hd = __shfl_sync(gm, d[M - 1], G - 1, G);
     hi = __shfl_sync(gm, i[M - 1], G - 1, G);
   }
