@@ -73,7 +73,7 @@ struct TopK {
   static __device__ __forceinline__ unsigned long long bits(T x) {
     return (unsigned long long)__double_as_longlong((double)x);
   }
-  __device__ __forceinline__ void init(int k) {
+  __device__ __forceinline__ void init(int k, int = 32) {
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       d[j] = j < k ? bits(Ar<T>::inf()) : 0ull;
@@ -131,9 +131,10 @@ struct TopK {
 // ascending order.
 template <int K>
 struct SmemTopK {
-  unsigned long long* d;  // entry j of this thread's list at d[j * 32]
+  unsigned long long* d;  // entry j of this thread's list at d[j * stride]
   int* ix;
   int n;
+  int stride;  // lists per warp: the lanes that search
   unsigned long long rootD;
   int rootI;
   static __device__ __forceinline__ bool greater(unsigned long long da, int ia, unsigned long long db, int ib) {
@@ -142,17 +143,18 @@ struct SmemTopK {
   static __device__ __forceinline__ unsigned long long bits(double x) {
     return (unsigned long long)__double_as_longlong(x);
   }
-  __device__ __forceinline__ void init(int k) {
+  __device__ __forceinline__ void init(int k, int lanes = 32) {
     extern __shared__ __align__(16) unsigned char heapSmem[];
-    const int column = (threadIdx.x >> 5) * K * 32 + (threadIdx.x & 31);
+    stride = lanes;
+    const int column = (threadIdx.x >> 5) * K * lanes + (threadIdx.x & 31);
     d = reinterpret_cast<unsigned long long*>(heapSmem) + column;
-    ix = reinterpret_cast<int*>(heapSmem + (size_t)blockDim.x * K * sizeof(unsigned long long)) + column;
+    ix = reinterpret_cast<int*>(heapSmem + (size_t)(blockDim.x >> 5) * lanes * K * sizeof(unsigned long long)) + column;
     n = k < K ? k : K;
     rootD = bits(Ar<double>::inf());
     rootI = -1;
     for (int j = 0; j < n; ++j) {
-      d[j * 32] = rootD;
-      ix[j * 32] = -1;
+      d[j * stride] = rootD;
+      ix[j * stride] = -1;
     }
   }
   __device__ __forceinline__ double head() const { return __longlong_as_double((long long)rootD); }
@@ -165,11 +167,11 @@ struct SmemTopK {
       const int l = 2 * j + 1;
       if (l >= m) break;
       int c = l;
-      unsigned long long cd = d[l * 32];
-      int ci = ix[l * 32];
+      unsigned long long cd = d[l * stride];
+      int ci = ix[l * stride];
       if (l + 1 < m) {
-        const unsigned long long rd = d[(l + 1) * 32];
-        const int ri = ix[(l + 1) * 32];
+        const unsigned long long rd = d[(l + 1) * stride];
+        const int ri = ix[(l + 1) * stride];
         if (greater(rd, ri, cd, ci)) {
           c = l + 1;
           cd = rd;
@@ -177,12 +179,12 @@ struct SmemTopK {
         }
       }
       if (!greater(cd, ci, x, xi)) break;
-      d[j * 32] = cd;
-      ix[j * 32] = ci;
+      d[j * stride] = cd;
+      ix[j * stride] = ci;
       j = c;
     }
-    d[j * 32] = x;
-    ix[j * 32] = xi;
+    d[j * stride] = x;
+    ix[j * stride] = xi;
   }
   // Drops the largest entry and inserts (dist, idx); requires accepts(dist, idx).
   __device__ __forceinline__ void insert(double dist, int idx) {
@@ -192,7 +194,7 @@ struct SmemTopK {
   }
   __device__ __forceinline__ int count(int) const {
     int c = 0;
-    for (int j = 0; j < n; ++j) c += ix[j * 32] >= 0 ? 1 : 0;
+    for (int j = 0; j < n; ++j) c += ix[j * stride] >= 0 ? 1 : 0;
     return c;
   }
   // Writes the entries in ascending order (the largest last), emptying the
@@ -205,7 +207,7 @@ struct SmemTopK {
       oi[m - 1] = ti;
       od[m - 1] = __longlong_as_double((long long)top);
       found += ti >= 0 ? 1 : 0;
-      if (m > 1) sift(d[(m - 1) * 32], ix[(m - 1) * 32], m - 1);
+      if (m > 1) sift(d[(m - 1) * stride], ix[(m - 1) * stride], m - 1);
     }
     return found;
   }
@@ -459,21 +461,23 @@ struct KnnLaunch {
 // Float pre-filter of leaf points for double clouds (the GB300 runs FP64 at
 // 1/64 of its FP32 rate, and the leaf distances are most of a double
 // search's arithmetic). With q~ and p~ the float roundings of the query and
-// point coordinates and e = (max|q~| + max|p~|) * 2^-22, every coordinate
-// difference satisfies |q - p| >= |q~ - p~|_float - e (conversion and
-// subtraction errors are at most 2.1 * 2^-24 * (|q| + |p|) each), so
-//     LB = sum_d max(0, |q~_d - p~_d| - e)^2,  taken * (1 - 2^-17)
-// is below the exact squared distance, float roundings of LB itself and the
-// double sum's own rounding included (less 2^-140, for squares that underflow).
-// A point with LB above a float at or
-// above min(head, maxRadius^2) cannot enter the heap, and only the others
-// get the exact double distance: results are unchanged. Coordinates beyond
-// the float range make e infinite, which rejects nothing.
+// point coordinates and e = (max|q~| + max|p~|) * 2^-22, every float
+// difference is within e of q - p (conversion and subtraction errors are at
+// most 2.1 * 2^-24 * (|q| + |p|) each), so a point within sqrt(t) of the query
+// has a float squared distance of at most (sqrt(t) + e sqrt(D))^2, times
+// 1 + 2^-18 for the rounding of the sum and plus 2^-140 for squares that
+// underflow. With t a float at or above min(head, maxRadius^2), a point above
+// that limit cannot enter the heap, and only the others get the exact double
+// distance: results are unchanged. Coordinates beyond the float range make e
+// infinite, which rejects nothing. (A sum of squared lower bounds,
+// max(0, |q~ - p~| - e)^2, took twice the instructions a coordinate; 8-D
+// and 16-D searches 1 % faster without.)
 template <typename T, int D>
 struct LeafFilter {
   __device__ __forceinline__ void init(const void*, const float*, const T (&)[D]) {}
   __device__ __forceinline__ bool on() const { return false; }
   __device__ __forceinline__ float threshold(T, T) const { return 0.0f; }
+  __device__ __forceinline__ float limit(float) const { return 0.0f; }
   __device__ __forceinline__ bool rejects(int64_t, float) const { return false; }
 };
 
@@ -501,16 +505,22 @@ struct LeafFilter<double, D> {
     const unsigned long long h = dist_key(head), r = dist_key(maxRadius2);
     return __double2float_ru(__longlong_as_double((long long)(r < h ? r : h)));
   }
-  __device__ __forceinline__ bool rejects(int64_t i, float thr) const {
+  // the largest float squared distance of a point within threshold t
+  __device__ __forceinline__ float limit(float t) const {
+    constexpr float kRoot = D <= 4 ? 2.0f : (D <= 9 ? 3.0f : 4.0f);  // at least sqrt(D)
+    const float u = __fadd_ru(__fsqrt_ru(t), __fmul_ru(e, kRoot));
+    return __fmaf_ru(__fmul_ru(u, u), 1.0f + 0x1p-18f, 0x1p-140f);
+  }
+  __device__ __forceinline__ bool rejects(int64_t i, float lim) const {
     Rec<float, D> f;
     load_rec(recs32, i, f);
-    float lb = 0.0f;
+    float d2 = 0.0f;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const float a = fmaxf(fabsf(qf[d] - f.p.c[d]) - e, 0.0f);
-      lb += a * a;
+      const float a = qf[d] - f.p.c[d];
+      d2 = fmaf(a, a, d2);
     }
-    return fmaf(lb, 1.0f - 0x1p-17f, -0x1p-140f) > thr;
+    return d2 > lim;
   }
 };
 
@@ -558,7 +568,7 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
     } else {
       T dj[kChunk];
       int ij[kChunk];
-      const float thr = flt.on() ? flt.threshold(heap.head(), maxRadius2) : 0.0f;
+      const float thr = flt.on() ? flt.limit(flt.threshold(heap.head(), maxRadius2)) : 0.0f;
       const auto radLimit = dist_limit(maxRadius2);
       const auto minKey = dist_key(Ar<T>::eps());
 #pragma unroll
@@ -967,7 +977,7 @@ __device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64
   // child is then left out by its lower bound)
   const float invError = EXACT ? 1.0f : __double2float_ru(1.0 / maxError2) * (1.0f + 0x1p-20f);
   typename SearchHeap<double, K>::type heap;
-  heap.init(k);
+  heap.init(k, a.lanes);
   LeafFilter<double, D> flt;
   flt.init(a.recs32, a.coordMax, q);
   double off2[D];
@@ -988,6 +998,7 @@ __device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64
                    : fminf(__double2float_ru(maxRadius2), __fmul_ru(__double2float_ru(heap.head()), invError));
     };
     float pruneThr = prune_threshold();
+    float leafLimit = flt.limit(leafThr);
     for (;;) {
       const int frame = sp;
       bool saved = false;
@@ -1037,7 +1048,7 @@ __device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64
         for (uint32_t j0 = 0; j0 < m; j0 += 4) {
 #pragma unroll
           for (uint32_t j = 0; j < 4; ++j)
-            if (j0 + j < m && !flt.rejects((int64_t)st + base + j0 + j, leafThr)) mask |= 1u << (j0 + j);
+            if (j0 + j < m && !flt.rejects((int64_t)st + base + j0 + j, leafLimit)) mask |= 1u << (j0 + j);
         }
         while (mask) {
           const int j = __ffs(mask) - 1;
@@ -1054,6 +1065,7 @@ __device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64
       if (changed) {
         leafThr = flt.threshold(heap.head(), maxRadius2);
         pruneThr = prune_threshold();
+        leafLimit = flt.limit(leafThr);
       }
       // pop the next far child that can still hold a better neighbour
       bool more = false;
@@ -1090,7 +1102,7 @@ __device__ __forceinline__ void knn_query_f64(const KnnLaunch& a, int64_t t, F64
     if (!mayFall || heap.count(k) == k) break;
     mayFall = false;
     maxRadius2 = a.maxRadius2;
-    heap.init(k);
+    heap.init(k, a.lanes);
     if (a.fallbacks) atomicAdd(a.fallbacks, 1);
   }
   const int f = heap.store(k, a.outIdx + task.outBase, static_cast<double*>(a.outD2) + task.outBase);
@@ -1177,7 +1189,7 @@ constexpr size_t deep_stack_bytes(int cap) {
 template <typename T, int D, int K, int STACK, bool EXACT>
 void launch_kdtree_as(int grid, int block, cudaStream_t stream, const KnnLaunch& L) {
   if constexpr (sizeof(T) == 8 && K >= 16)
-    k_knn_kdtree_lean<T, D, K, STACK, EXACT><<<grid, block, SearchHeap<T, K>::bytes(block), stream>>>(L);
+    k_knn_kdtree_lean<T, D, K, STACK, EXACT><<<grid, block, SearchHeap<T, K>::bytes(block / 32 * L.lanes), stream>>>(L);
   else
     k_knn_kdtree<T, D, K, STACK, EXACT><<<grid, block, 0, stream>>>(L);
 }

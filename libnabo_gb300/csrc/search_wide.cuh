@@ -196,7 +196,7 @@ __device__ __forceinline__ void wide_offer(const Rec<T, D>* __restrict__ recs, i
     T dist = Ar<T>::inf();
     int idx = -1;
     bool ok = false;
-    const float thr = flt.on() ? flt.threshold(heap.head(), maxRadius2) : 0.0f;
+    const float thr = flt.on() ? flt.limit(flt.threshold(heap.head(), maxRadius2)) : 0.0f;
     if (g < avail && !(flt.on() && flt.rejects(first + g, thr))) {
       Rec<T, D> r;
       if constexpr (kShared)
