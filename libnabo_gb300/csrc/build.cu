@@ -256,30 +256,10 @@ __device__ __forceinline__ int arg_max_extent(const T* lo, const T* hi, int dim)
 }
 
 // Median-split trees (split rule 1): the cut is just above the median of the
-// segment's coordinates along the cut dimension (sampled at kMedianSamples
-// evenly spaced positions at the level-synchronous levels, where the
-// segment's points are in no particular order; exact below kHeld points, in
-// k_mid). Just above
-// (the next representable value): points equal to the median go left and
-// hardly any point lies on the cut, so the build's second partition pass,
-// which only segments with points on their cut run, is skipped.
-template <typename T>
-__device__ T sampled_median(const T* __restrict__ val, int start, int count) {
-  T smp[kMedianSamples];
-  for (int j = 0; j < kMedianSamples; ++j)
-    smp[j] = val[start + (int)((int64_t)(2 * j + 1) * count / (2 * kMedianSamples))];
-  for (int i = 1; i < kMedianSamples; ++i) {  // insertion sort
-    const T x = smp[i];
-    int j = i - 1;
-    while (j >= 0 && x < smp[j]) {
-      smp[j + 1] = smp[j];
-      --j;
-    }
-    smp[j + 1] = x;
-  }
-  return smp[kMedianSamples / 2];
-}
-
+// segment's coordinates along the cut dimension (of kMedianSamples values at
+// evenly spaced positions, the segment's points being in no particular order;
+// exact up to kHeld points, in k_mid). Just above (the next representable
+// value): points equal to the median go left and hardly any lies on the cut.
 // Single block: exclusive scan of the per-block sums; the grand total goes
 // to *total. Each thread scans a contiguous run serially and one block-wide
 // scan joins the runs (a loop of block-wide scans over the sums would
@@ -469,12 +449,21 @@ __device__ __forceinline__ int2 median_flag(const SegLevel<T>& L, int s, T v) {
   return make_int2(v <= m ? 1 : 0, v < m ? 1 : 0);
 }
 
+// Each segment's sampled median, a warp each. (A thread each, sorting its 31
+// samples in local memory, took 25 us a level; at the 256-point handover the
+// levels had ten times the segments and warps were slower.)
 template <typename T, int D>
 __global__ void k_median_cut(SegLevel<T> L, const LevelState* st, MedianBufs<T, D> B) {
   pdl_begin();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  using Key = typename KeyOf<T>::type;
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (s >= st->nseg) return;
-  L.cut[s] = sampled_median(B.vals(st->level & 1), L.start[s], L.count[s]);
+  const T* val = B.vals(st->level & 1) + L.start[s];
+  const int64_t count = L.count[s];
+  Key e[1] = {lane < kMedianSamples ? ordered_key(val[(2 * lane + 1) * count / (2 * kMedianSamples)]) : ~Key(0)};
+  warp_sort_keys<1>(e, lane);
+  if (lane == kMedianSamples / 2) L.cut[s] = ordered_val(e[0], T(0));
 }
 
 // Block b scans tiles [b * tiles, (b + 1) * tiles) in position order and
@@ -1246,7 +1235,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
         if (nseg == 0) break;
         if (level >= N) return set_error(kErrInternal, "kd-tree build: more levels than points");
       }
-      NABO_CUDA_TRY(launch_pdl(k_median_cut<T, D>, sg, 128, 0, stream, cur, st, mb));
+      NABO_CUDA_TRY(launch_pdl(k_median_cut<T, D>, ceil_div(segCap, 4), 128, 0, stream, cur, st, mb));
       NABO_CUDA_TRY(launch_pdl(k_median_sums<T, D>, mBlocks, kBlock, 0, stream, mb, nPad, cur, mTiles, blockSums,
                                segFirst, segLast, st));
       NABO_CUDA_TRY(launch_pdl(k_scan_block_sums, 1, kBlock, 0, stream, blockSums, mBlocks, passTotal, st));
