@@ -698,18 +698,16 @@ __device__ __forceinline__ T warp_sampled_median(const Rec<T, D>* node, int coun
 // every 32nd of them in each lane: bit by bit below the bits that all keys
 // share, until one candidate is left (about 11 rounds instead of a bit each).
 constexpr int kHeld = 256;
-template <typename T, int D>
-__device__ __forceinline__ T warp_median(const Rec<T, D>* node, int count, int cd, int lane) {
+template <int kPer, typename T, int D>
+__device__ __forceinline__ T warp_median_of(const Rec<T, D>* node, int count, int cd, int lane) {
   using Key = typename KeyOf<T>::type;
-  constexpr int kPer = kHeld / 32;
-  const int held = (count + 31) >> 5;
   Key k[kPer];
   Key any = 0, all = ~Key(0);
   unsigned alive = 0;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     k[j] = 0;
-    if (j < held && lane + 32 * j < count) {
+    if (lane + 32 * j < count) {
       k[j] = ordered_key(node[lane + 32 * j].p.c[cd]);
       any |= k[j];
       all &= k[j];
@@ -741,6 +739,12 @@ __device__ __forceinline__ T warp_median(const Rec<T, D>* node, int count, int c
     if ((alive & ((1u << j) - 1u)) == 0u) m = k[j];
   const int src = __ffs(__ballot_sync(kFull, alive != 0u)) - 1;
   return ordered_val(__shfl_sync(kFull, m, src), T(0));
+}
+template <typename T, int D>
+__device__ __forceinline__ T warp_median(const Rec<T, D>* node, int count, int cd, int lane) {
+  if (count <= 64) return warp_median_of<2>(node, count, cd, lane);
+  if (count <= 128) return warp_median_of<4>(node, count, cd, lane);
+  return warp_median_of<kHeld / 32>(node, count, cd, lane);
 }
 
 // Splits a node, by a warp, at `ideal` (the median rule: just above it, so
