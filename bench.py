@@ -626,10 +626,12 @@ def run_batched(args):
         "cpu_baseline": None if base is None else {kk: base[kk] for kk in ("value", "unit", "cores", "kind",
                                                                            "sample", "search_only_queries_per_s")},
         "clocks": clk.summary(),
-        # per graph launch: forest set-up 6 + 17 per level + small/status/
-        # renumber/copy 4; search: leaf cells, 3 scan kernels, placement,
-        # run sort, search 7
-        "gpu_launches": args.steps * (6 + 17 * choice["maxLevels"] + 4 + 7),
+        # per graph launch: keys, bounds, roots; the top levels (the median
+        # rule 6 launches a level, the first ids and the flush; the
+        # reference's rule one launch); small segments, 2 for the leaf
+        # ranks, nodes; search: leaf cells, 5 of ordering, run sort, a search
+        # for each of the 3 values of k and one for tall trees
+        "gpu_launches": args.steps * (3 + (2 + 6 * choice["maxLevels"] if choice.get("splitRule") else 1) + 4 + 11),
     }
     print(json.dumps(res))
     if world > 1:
@@ -899,8 +901,9 @@ def run_c4(args):
 # ---------------------------------------------------------------------------
 # Brute force: 100,000 uniform 3-D float32 points against 100,000 queries,
 # k = 5 (the reference's small case scaled up so one launch is measurable).
-# Bound by the FP32 pipe: flops = Q * N * 3D (D subtractions and D
-# multiply-adds counted as two), against the FMA peak measured live.
+# flops = Q * N * 3D (D subtractions and D multiply-adds counted as two),
+# against the FP32 FMA peak measured live; the float search filters the pairs
+# on the tensor cores first, so this is a rate of useful work, not of a pipe.
 
 BF_METRIC = "brute-force kNN queries/s (100k uniform 3-D points, k=5)"
 
@@ -955,17 +958,19 @@ def run_bf(args):
         "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": "bruteforce_uniform_100k_k5", "points": n, "queries": nq, "k": k,
-                   "l2": "cloud (1.6 MB) is reread from L2 by design; the bound is the FP32 pipe"},
+                   "l2": "cloud (1.6 MB) is reread from L2 by design"},
         "e2e": {"value": nq / e2e_s, "unit": "queries/s", "h2d_bytes_per_step": int(q.nbytes),
                 "d2h_bytes_per_step": int(nq * k * 8)},
         "roofline": {"bound": "fp32 pipe", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": None, "peak_source": "FMA chains measured in this run",
-                     "kernel": "k_knn_bruteforce", "kernel_ms": kernel_ms, "flops_per_launch": flops},
+                     "kernel": "k_bf_tc (with its operand and merge launches)", "kernel_ms": kernel_ms,
+                     "flops_per_launch": flops},
         "exact_vs_oracle": {"queries_checked": sample,
                             "identical": bool(np.array_equal(gi, oi) and np.array_equal(gd, od))},
         "cpu_baseline": {"value": sample / cpu_s, "unit": "queries/s", "cores": O.num_threads(), "kind": "port",
                          "sample": f"{sample} queries against all {n} points (oracle brute force)"},
-        "clocks": clk.summary(), "gpu_launches": args.steps,
+        # the points' operand, the search, and the merge of its block rows
+        "clocks": clk.summary(), "gpu_launches": 3 * args.steps,
     }
     # the same search in double: bound by the FP64 pipe (1/64 of the FP32
     # rate on this GPU), so fewer queries

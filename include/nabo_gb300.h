@@ -287,8 +287,8 @@ int nabo_cuda_radius_model_set(nabo_cuda_radius_model* m, const float* params, c
  * local to the cloud. */
 typedef struct nabo_cuda_batch nabo_cuda_batch; /* opaque */
 
-/* maxLevels: levels of the level-synchronous top build (segments of more
- * than 256 points), run without host synchronisation (0 = 48). A tree
+/* maxLevels: levels at which a segment of more than 256 points may be
+ * split (0 = 48); the build runs without host synchronisation. A tree
  * needing more is reported by nabo_cuda_batch_status. params: bucketSize
  * and threadsPerBlock (may be NULL). */
 int nabo_cuda_batch_create(int dtype, int dim, int nClouds, const int64_t* pointCounts,

@@ -260,6 +260,7 @@ __device__ __forceinline__ int arg_max_extent(const T* lo, const T* hi, int dim)
 // evenly spaced positions, the segment's points being in no particular order;
 // exact up to kHeld points, in k_mid). Just above (the next representable
 // value): points equal to the median go left and hardly any lies on the cut.
+
 // Single block: exclusive scan of the per-block sums; the grand total goes
 // to *total. Each thread scans a contiguous run serially and one block-wide
 // scan joins the runs (a loop of block-wide scans over the sums would
@@ -449,9 +450,10 @@ __device__ __forceinline__ int2 median_flag(const SegLevel<T>& L, int s, T v) {
   return make_int2(v <= m ? 1 : 0, v < m ? 1 : 0);
 }
 
-// Each segment's sampled median, a warp each. (A thread each, sorting its 31
-// samples in local memory, took 25 us a level; at the 256-point handover the
-// levels had ten times the segments and warps were slower.)
+// Each segment's sampled median, a warp each: latency-bound, one load and a
+// shuffle sort. (A thread each, sorting its 31 samples in local memory, took
+// 340 us of a 512-cloud, 22 M-point build; this takes 92. With the handover
+// at 256 points the levels had ten times the segments and warps were slower.)
 template <typename T, int D>
 __global__ void k_median_cut(SegLevel<T> L, const LevelState* st, MedianBufs<T, D> B) {
   pdl_begin();
@@ -1342,8 +1344,6 @@ int build_kdtree(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   }
   if (stats) {
     stats->topLevels = hs[3];
-    stats->topNodes = 0;
-    stats->smallSegments = 0;
   }
   return kOk;
 }

@@ -697,6 +697,8 @@ __device__ __forceinline__ T warp_sampled_median(const Rec<T, D>* node, int coun
 // The lower median (rank count / 2) of up to kHeld values, by a warp holding
 // every 32nd of them in each lane: bit by bit below the bits that all keys
 // share, until one candidate is left (about 11 rounds instead of a bit each).
+// Instantiated for 64, 128 and 256 values: most nodes have far fewer than 256
+// (k_mid of a 512-cloud, 22 M-point build: 2.75 -> 2.64 ms).
 constexpr int kHeld = 256;
 template <int kPer, typename T, int D>
 __device__ __forceinline__ T warp_median_of(const Rec<T, D>* node, int count, int cd, int lane) {

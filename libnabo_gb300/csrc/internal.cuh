@@ -104,9 +104,7 @@ struct DeviceCloud {
 };
 
 struct BuildStats {
-  int topLevels = 0;
-  int64_t topNodes = 0;
-  int64_t smallSegments = 0;
+  int topLevels = 0;  // levels split before the small segments' phase
 };
 
 // Builds the kd-tree of `n` points (dim coordinates each, column stride

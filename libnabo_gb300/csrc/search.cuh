@@ -121,8 +121,9 @@ struct TopK {
 
 // double lists of 16 or more entries in the kd-tree search: a binary
 // max-heap of (dist2 bits, index) in (dynamic) shared memory, a section per
-// warp, slot-major with one column per lane, the root kept in registers for
-// the accept test. Held in registers, such a list (3
+// warp, slot-major with one column per searching lane (a call that spreads few
+// queries over many warps asks for less shared memory: 6000 queries, 8-D,
+// k = 32, 3.50 -> 3.35 ms), the root kept in registers for the accept test. Held in registers, such a list (3
 // registers an entry) spilled under the search kernel's register cap, and
 // every insertion walked the spilled entries through local memory (8-D,
 // k = 32: 2.2 G local loads a launch). Here an insertion sifts down at most
@@ -1145,10 +1146,10 @@ __global__ void __launch_bounds__(128) k_knn_kdtree(KnnLaunch a) {
   knn_kdtree_body<T, D, K, STACK, EXACT>(a);
 }
 
-// Double searches with a long top-k hold ~100 registers of heap alone;
-// limited to 128 registers a thread, 4 blocks share an SM, and the FP64 pipe
-// gets the extra warps it needs to hide its latency (12 % faster on 8-D
-// clouds, k = 32).
+// Double searches of 16 or more neighbours: limited to 128 registers a
+// thread, so that 4 blocks share an SM (their lists are in shared memory,
+// SmemTopK) and more warps hide each other's loads from L2, which bound the
+// kernel.
 template <typename T, int D, int K, int STACK, bool EXACT>
 __global__ void __launch_bounds__(128, 4) k_knn_kdtree_lean(KnnLaunch a) {
   knn_kdtree_body<T, D, K, STACK, EXACT>(a);
