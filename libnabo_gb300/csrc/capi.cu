@@ -85,9 +85,22 @@ cudaError_t object_alloc(void** p, size_t bytes, cudaStream_t stream) {
   return e == cudaSuccess ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : e;
 }
 
+// Waits for all work on the device by freeing a small cudaMalloc block (2 us
+// when idle). cudaDeviceSynchronize would break a stream capture that another
+// thread has open; cudaFree does not.
+static cudaError_t wait_for_device() {
+  void* p = nullptr;
+  const cudaError_t e = cudaMalloc(&p, 256);
+  if (e == cudaSuccess) return cudaFree(p);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return cudaDeviceSynchronize();
+}
+
 cudaError_t object_free(void* const* p, int count) {
   cudaMemPool_t pool;
-  cudaError_t e = cudaDeviceSynchronize();
+  cudaError_t e = wait_for_device();
+  if (e != cudaSuccess) return e;  // still in use, for all we know: not freed (as with a failing cudaFree)
   const cudaError_t pe = library_pool(&pool);
   for (int i = 0; i < count; ++i) {
     const cudaError_t fe = p[i] ? cudaFreeAsync(p[i], cudaStreamPerThread) : cudaSuccess;
