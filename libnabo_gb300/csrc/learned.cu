@@ -91,8 +91,9 @@ __device__ __forceinline__ float silu_fast(float z) {
 }
 
 // Occupancies of scales [s0, s0 + n) for point p: the first probe of every
-// scale is issued before any is inspected (independent loads in flight);
-// collisions continue with the bounded linear probe.
+// scale, key and count, is issued before any is inspected (independent loads
+// in flight; the count only after its key had matched: k_mlp_radius 110 -> 102
+// us at 1.15 M queries); collisions continue with the bounded linear probe.
 template <int N>
 __device__ __forceinline__ void voxel_counts(const FeatureSpace& fs, int s0, const float (&p)[3], float (&out)[N]) {
   unsigned long long key[N];
@@ -114,15 +115,19 @@ __device__ __forceinline__ void voxel_counts(const FeatureSpace& fs, int s0, con
     slot[j] = (uint32_t)mix64(key[j]) & fs.mask[s];
   }
   unsigned long long k0[N];
+  uint32_t c0[N];
 #pragma unroll
-  for (int j = 0; j < N; ++j) k0[j] = inside[j] ? __ldg(fs.keys[s0 + j] + slot[j]) : 0ull;
+  for (int j = 0; j < N; ++j) {
+    k0[j] = inside[j] ? __ldg(fs.keys[s0 + j] + slot[j]) : 0ull;
+    c0[j] = inside[j] ? __ldg(fs.counts[s0 + j] + slot[j]) : 0u;
+  }
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     const int s = s0 + j;
     uint32_t cnt = 0u;
     if (inside[j] && k0[j] != 0ull) {
       if (k0[j] == key[j]) {
-        cnt = __ldg(fs.counts[s] + slot[j]);
+        cnt = c0[j];
       } else {
         const uint32_t mask = fs.mask[s];
         uint32_t sl = (slot[j] + 1u) & mask;
@@ -429,24 +434,45 @@ struct RadiusOut {
 };
 
 constexpr int kInferWarps = 8;
+// Blocks per SM, one wave of them, so that a block stages the weights once
+// (2, 3, 4: 115, 110, 106 us; with the counts loaded early 102 by 3, 104 by 4).
+constexpr int kInferBlocks = 3;
 
-// The network's weights in shared memory.
+// The network's weights in shared memory, as the lanes of a warp read them: a
+// B operand of m16n8k16 is two words per lane, and a lane's words for a whole
+// n-tile of layer 2 are two 16-byte reads without bank conflicts. (Rows of
+// words, read a word at a time, collided 8 ways. k_mlp_radius, 1.15 M queries:
+// 189 us, 110 with these layouts and one wave of blocks; what is left is the
+// voxel probes' latency and instruction issue.)
 struct InferSmem {
-  __nv_bfloat16 W1[kH * kF];
-  __nv_bfloat16 W2[kH * kH];
-  float b1[kH], b2[kH], w3[kH];
+  uint2 W1[kH / 8][32];     // n-tile: k 0-7, 8-15
+  uint4 W2[kH / 8][2][32];  // n-tile, pair of k-steps: {k 0-7, 8-15} of either
+  float2 b1[kH / 2], b2[kH / 2], w3[kH / 2];
   float b3;
-  __nv_bfloat16 X[kInferWarps][16 * kF];
+  uint4 X[kInferWarps][2][16];  // inputs 0-7 and 8-15 of each row, BF16
 };
+static_assert(kF == 16 && kH == 64, "the layouts below");
 
 __device__ __forceinline__ void stage_weights(InferSmem& sm, const __nv_bfloat16* __restrict__ Wb) {
+  static_assert(kOffW1 % 2 == 0 && kOffW2 % 2 == 0, "weights read in pairs");
   const int tid = threadIdx.x;
-  for (int i = tid; i < kH * kF; i += blockDim.x) sm.W1[i] = Wb[kOffW1 + i];
-  for (int i = tid; i < kH * kH; i += blockDim.x) sm.W2[i] = Wb[kOffW2 + i];
-  for (int i = tid; i < kH; i += blockDim.x) {
-    sm.b1[i] = __bfloat162float(Wb[kOffB1 + i]);
-    sm.b2[i] = __bfloat162float(Wb[kOffB2 + i]);
-    sm.w3[i] = __bfloat162float(Wb[kOffW3 + i]);
+  const uint32_t* W1w = reinterpret_cast<const uint32_t*>(Wb + kOffW1);  // row j = 8 words
+  const uint32_t* W2w = reinterpret_cast<const uint32_t*>(Wb + kOffW2);  // row j = 32 words
+  for (int i = tid; i < kH / 8 * 32; i += blockDim.x) {
+    const uint32_t* w = W1w + (8 * (i >> 5) + ((i & 31) >> 2)) * 8 + (i & 3);
+    sm.W1[i >> 5][i & 31] = make_uint2(w[0], w[4]);
+  }
+  for (int i = tid; i < kH / 8 * 64; i += blockDim.x) {
+    const uint32_t* w = W2w + (8 * (i >> 6) + ((i & 31) >> 2)) * 32 + 16 * ((i >> 5) & 1) + (i & 3);
+    sm.W2[i >> 6][(i >> 5) & 1][i & 31] = make_uint4(w[0], w[4], w[8], w[12]);
+  }
+  for (int i = tid; i < kH / 2; i += blockDim.x) {
+    auto pair = [&](int off) {
+      return make_float2(__bfloat162float(Wb[off + 2 * i]), __bfloat162float(Wb[off + 2 * i + 1]));
+    };
+    sm.b1[i] = pair(kOffB1);
+    sm.b2[i] = pair(kOffB2);
+    sm.w3[i] = pair(kOffW3);
   }
   if (tid == 0) sm.b3 = __bfloat162float(Wb[kOffB3]);
 }
@@ -458,20 +484,19 @@ template <typename T>
 __device__ __forceinline__ void mlp_tile(const InferSmem& sm, int warp, int lane, int64_t q0, int64_t nq,
                                          const RadiusOut& ro, T* radii, float* rawOut) {
   const int g = lane >> 2, tig = lane & 3;
-  const uint32_t* X32 = reinterpret_cast<const uint32_t*>(sm.X[warp]);  // row = 8 words
+  const uint32_t* X32 = reinterpret_cast<const uint32_t*>(sm.X[warp]);  // half of a row = 4 words
   uint32_t a[4];
-  a[0] = X32[g * 8 + tig];
-  a[1] = X32[(g + 8) * 8 + tig];
-  a[2] = X32[g * 8 + 4 + tig];
-  a[3] = X32[(g + 8) * 8 + 4 + tig];
+  a[0] = X32[g * 4 + tig];
+  a[1] = X32[(g + 8) * 4 + tig];
+  a[2] = X32[64 + g * 4 + tig];
+  a[3] = X32[64 + (g + 8) * 4 + tig];
   // layer 1: 8 n-tiles of 8 hidden units
-  const uint32_t* W1w = reinterpret_cast<const uint32_t*>(sm.W1);  // row j = 8 words
   float z1[8][4];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     z1[j][0] = z1[j][1] = z1[j][2] = z1[j][3] = 0.0f;
-    const int n = 8 * j + g;
-    mma16816(z1[j], a, W1w[n * 8 + tig], W1w[n * 8 + 4 + tig]);
+    const uint2 w = sm.W1[j][lane];
+    mma16816(z1[j], a, w.x, w.y);
   }
   // SiLU, BF16, repacked as the A operand of layer 2 (4 k-steps); fragment
   // order for m16n8k16 A: {row g k0-7, row g+8 k0-7, row g k8-15, row g+8
@@ -482,36 +507,35 @@ __device__ __forceinline__ void mlp_tile(const InferSmem& sm, int warp, int lane
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int j = 2 * s + h;
-      const int c = 8 * j + 2 * tig;
+      const float2 b = sm.b1[4 * j + tig];
       float v[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float z = z1[j][e] + sm.b1[c + (e & 1)];
-        v[e] = silu_fast(z);
-      }
+      for (int e = 0; e < 4; ++e) v[e] = silu_fast(z1[j][e] + (e & 1 ? b.y : b.x));
       A2[s][2 * h + 0] = pack2(v[0], v[1]);
       A2[s][2 * h + 1] = pack2(v[2], v[3]);
     }
   }
   // layer 2
-  const uint32_t* W2w = reinterpret_cast<const uint32_t*>(sm.W2);  // row j = 32 words
   float z2[8][4];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     z2[j][0] = z2[j][1] = z2[j][2] = z2[j][3] = 0.0f;
-    const int n = 8 * j + g;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) mma16816(z2[j], A2[s], W2w[n * 32 + 8 * s + tig], W2w[n * 32 + 8 * s + 4 + tig]);
+    for (int p = 0; p < 2; ++p) {
+      const uint4 w = sm.W2[j][p][lane];
+      mma16816(z2[j], A2[2 * p], w.x, w.y);
+      mma16816(z2[j], A2[2 * p + 1], w.z, w.w);
+    }
   }
   // output layer: rows g and g+8
   float y0 = 0.0f, y1 = 0.0f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const int c = 8 * j + 2 * tig;
+    const float2 b = sm.b2[4 * j + tig], w = sm.w3[4 * j + tig];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float z = z2[j][e] + sm.b2[c + (e & 1)];
-      const float act = silu_fast(z) * sm.w3[c + (e & 1)];
+      const float z = z2[j][e] + (e & 1 ? b.y : b.x);
+      const float act = silu_fast(z) * (e & 1 ? w.y : w.x);
       if (e < 2)
         y0 += act;
       else
@@ -538,8 +562,12 @@ __device__ __forceinline__ void mlp_tile(const InferSmem& sm, int warp, int lane
   }
 }
 
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kInferWarps * 32) k_mlp_radius(const T* __restrict__ query, int64_t nq,
+__global__ void __launch_bounds__(kInferWarps * 32, kInferBlocks) k_mlp_radius(const T* __restrict__ query, int64_t nq,
                                                                  int64_t qStride, FeatureSpace fs,
                                                                  const __nv_bfloat16* __restrict__ Wb, RadiusOut ro,
                                                                  T* radii, float* rawOut) {
@@ -551,39 +579,39 @@ __global__ void __launch_bounds__(kInferWarps * 32) k_mlp_radius(const T* __rest
   for (int64_t tile = (int64_t)blockIdx.x * kInferWarps + warp; tile < tiles; tile += (int64_t)gridDim.x * kInferWarps) {
     const int64_t q0 = tile * 16;
     // features of the tile's 16 queries: lanes l and l + 16 share query l;
-    // the first lane writes the coordinates and the finer half of the voxel
-    // scales, the second the coarser half
+    // the first lane writes inputs 0-7 (the coordinates, then the voxel
+    // scales from the finest), the second 8-15, each probing half the scales
     {
-      const int row = lane & 15;
-      const bool second = lane >= 16;
+      const int row = lane & 15, half = lane >> 4;
       const int64_t qi = q0 + row;
-      __nv_bfloat16* xr = sm.X[warp] + row * kF;
-      if (qi < nq) {
-        const T* qp = query + qi * qStride;
-        if (fs.useGrid) {
+      const bool live = qi < nq;
+      const T* qp = query + qi * qStride;
+      float v[8] = {};
+      if (fs.useGrid) {
+        static_assert(kScales == 8, "inputs 3-10");
+        float occ[4] = {};
+        if (live) {
           const float p[3] = {(float)qp[0], (float)qp[1], (float)qp[2]};
-          float occ[kScales / 2];
-          voxel_counts<kScales / 2>(fs, second ? kScales / 2 : 0, p, occ);
-#pragma unroll
-          for (int j = 0; j < kScales / 2; ++j) xr[3 + (second ? kScales / 2 : 0) + j] = __float2bfloat16_rn(occ[j]);
-          if (!second) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              xr[d] = __float2bfloat16_rn(fminf(fmaxf(((float)qp[d] - fs.center[d]) * fs.invHalf[d], -4.f), 4.f));
-          } else {
-#pragma unroll
-            for (int j = 3 + kScales; j < kF; ++j) xr[j] = __float2bfloat16_rn(0.0f);
-          }
-        } else if (!second) {
-          float f[kF];
-          features(qp, fs, f);
-#pragma unroll
-          for (int j = 0; j < kF; ++j) xr[j] = __float2bfloat16_rn(f[j]);
+          voxel_counts<4>(fs, 4 * half, p, occ);
         }
-      } else if (!second) {
+        const float fifth = __shfl_xor_sync(0xffffffffu, occ[0], 16);  // the first lane's: input 7
+        if (live && half == 0) {
 #pragma unroll
-        for (int j = 0; j < kF; ++j) xr[j] = __float2bfloat16_rn(0.0f);
+          for (int d = 0; d < 3; ++d) v[d] = fminf(fmaxf(((float)qp[d] - fs.center[d]) * fs.invHalf[d], -4.f), 4.f);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[3 + j] = occ[j];
+          v[7] = fifth;
+        } else if (live) {
+#pragma unroll
+          for (int j = 1; j < 4; ++j) v[j - 1] = occ[j];
+        }
+      } else if (live) {
+        float f[kF];
+        features(qp, fs, f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = half ? f[8 + j] : f[j];
       }
+      sm.X[warp][half][row] = pack8(v);
     }
     __syncwarp();
     mlp_tile<T>(sm, warp, lane, q0, nq, ro, radii, rawOut);
@@ -727,7 +755,6 @@ __global__ void __launch_bounds__(kInferWarps * 32) k_mlp_radius_batch(const T* 
     const int64_t q0 = tile * 16;
     if (lane < 16) {
       const int64_t qi = q0 + lane;
-      __nv_bfloat16* xr = sm.X[warp] + lane * kF;
       float f[kBatchInputs];
       if (qi < nq) {
         batch_raw_features<T, D>(query + qi * bf.dim, qi, bf, f);
@@ -735,8 +762,12 @@ __global__ void __launch_bounds__(kInferWarps * 32) k_mlp_radius_batch(const T* 
 #pragma unroll
         for (int j = 0; j < kBatchInputs; ++j) f[j] = fs.center[j];
       }
+      static_assert(kBatchInputs == 8, "the first half of a row");
+      float v[8];
 #pragma unroll
-      for (int j = 0; j < kF; ++j) xr[j] = __float2bfloat16_rn(batch_input(f, fs, j));
+      for (int j = 0; j < 8; ++j) v[j] = batch_input(f, fs, j);
+      sm.X[warp][0][lane] = pack8(v);
+      sm.X[warp][1][lane] = make_uint4(0u, 0u, 0u, 0u);
     }
     __syncwarp();
     mlp_tile<T>(sm, warp, lane, q0, nq, ro, radii, rawOut);
@@ -854,7 +885,7 @@ int launch_radius(const RadiusModel& m, const void* query, int64_t nq, int64_t q
   ro.margin = m.margin;
   ro.maxRadius = maxRadius;
   const int64_t tiles = (nq + 15) / 16;
-  const int grid = (int)std::min<int64_t>(ceil_div(tiles, kInferWarps), 152 * 16);
+  const int grid = (int)std::min<int64_t>(ceil_div(tiles, kInferWarps), 152 * kInferBlocks);
   if (m.dtype == NABO_CUDA_FLOAT32)
     k_mlp_radius<float><<<grid, kInferWarps * 32, 0, st>>>(static_cast<const float*>(query), nq, qStride, m.fs, m.pb,
                                                              ro, static_cast<float*>(radii), raw);
