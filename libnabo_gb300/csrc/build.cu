@@ -1085,7 +1085,11 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   // points 18.8 ms, 1024 18.3, 2048 18.1, 4096 17.9.)
   const int smallMax = Mid::kMax;
   const size_t midSmem = Mid::smem(smallMax, bucket);
-  NABO_CUDA_TRY(cudaFuncSetAttribute(k_mid<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)midSmem));
+  // The limit is the kernel's, shared by all threads that build: always set to
+  // the most any build asks for (the smallest bucket's), never to this one's
+  // own need, which could refuse another thread's launch.
+  constexpr int kMidSmemMax = (int)Mid::smem(Mid::kMax, 2);
+  NABO_CUDA_TRY(cudaFuncSetAttribute(k_mid<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmemMax));
   int midOcc = 0;
   NABO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&midOcc, k_mid<T, D>, Mid::kThreads, midSmem));
 
@@ -1209,7 +1213,9 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
                          : topMode == kTopLists  ? (const void*)k_top<T, D, kTopLists>
                                                  : (const void*)k_top<T, D, kTopGlobal>;
     const size_t topSmem = topMode == kTopResident ? withRecs : (topMode == kTopLists ? withLists : 0);
-    NABO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)topSmem));
+    // the most any build asks for, as k_mid's
+    if (topSmem > 0)
+      NABO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmemMax));
     void* args[] = {&ta};
     NABO_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(topBlocks), dim3(kTopThreads), args, topSmem, stream));
   }

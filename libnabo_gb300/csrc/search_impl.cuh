@@ -63,9 +63,10 @@ int launch_wide_kdtree_as(const KnnLaunch& L, int height, cudaStream_t stream) {
   const size_t smem = wide_stack_bytes<T, D>(threads / G, cap);
   if (smem > kWideSmemMax) return kNeedsSlab;
   cudaError_t e = cudaSuccess;
+  // (the most any search asks for: the limit is shared by all threads' searches)
   if (smem > 48 * 1024)
     e = cudaFuncSetAttribute(k_knn_kdtree_wide<T, D, M, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+                             (int)kWideSmemMax);
   if (e != cudaSuccess) return cuda_error(e, "wide kd-tree search shared memory");
   const int grid = ceil_div(L.nq, threads / G);
   k_knn_kdtree_wide<T, D, M, G><<<grid, threads, smem, stream>>>(L, cap);
