@@ -126,7 +126,10 @@ int nabo_cuda_create_device(int dtype, const void* cloud, int rows, int64_t n, i
                             int searchType, unsigned creationFlags, const nabo_cuda_params* params,
                             nabo_cuda_search** out);
 
-/* Releases the object and its device memory. Accepts NULL.
+/* Releases the object and its device memory, waiting for the device; a stream
+ * capture open in this or another thread stays valid. Accepts NULL. On an
+ * error the memory that could not be given back and the handle stay, and the
+ * call may be repeated.
  * Replaces the virtual destructor (nabo/nabo.h:427). */
 int nabo_cuda_destroy(nabo_cuda_search* s);
 

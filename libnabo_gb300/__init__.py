@@ -188,7 +188,7 @@ class NearestNeighbourSearch:
     def close(self) -> None:
         h = getattr(self, "_h", None)
         if h is not None and h.value:
-            _lib.nabo_cuda_destroy(h)
+            _check(_lib.nabo_cuda_destroy(h))
             self._h = ctypes.c_void_p()
 
     def __del__(self):

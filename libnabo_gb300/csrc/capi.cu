@@ -85,10 +85,24 @@ cudaError_t object_alloc(void** p, size_t bytes, cudaStream_t stream) {
   return e == cudaSuccess ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : e;
 }
 
+namespace {
+
+// While it lives, this thread may make the calls that a stream capture forbids
+// (cudaMalloc, cudaFree) without invalidating a capture that this thread or,
+// in the global mode, another one has open.
+struct OutsideCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Waits for all work on the device by freeing a small cudaMalloc block (2 us
-// when idle). cudaDeviceSynchronize would break a stream capture that another
-// thread has open; cudaFree does not.
-static cudaError_t wait_for_device() {
+// when idle): cudaDeviceSynchronize would break an open stream capture, in
+// whatever mode. That cudaFree waits is its behaviour rather than its contract
+// (measured: 4.8 ms behind a 5 ms kernel); a plain cudaFree of memory that
+// searches still read relies on the same.
+cudaError_t wait_for_device() {
+  const OutsideCapture outside;
   void* p = nullptr;
   const cudaError_t e = cudaMalloc(&p, 256);
   if (e == cudaSuccess) return cudaFree(p);
@@ -97,21 +111,41 @@ static cudaError_t wait_for_device() {
   return cudaDeviceSynchronize();
 }
 
-cudaError_t object_free(void* const* p, int count) {
+// The library's own stream on the current device for giving memory back (a
+// caller may be capturing any other).
+std::mutex g_freeStreamMutex;
+cudaStream_t g_freeStreams[64] = {};
+cudaError_t free_stream(cudaStream_t* stream) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(g_freeStreamMutex);
+  if (!g_freeStreams[dev]) e = cudaStreamCreateWithFlags(&g_freeStreams[dev], cudaStreamNonBlocking);
+  *stream = g_freeStreams[dev];
+  return e;
+}
+
+}  // namespace
+
+cudaError_t object_free(void** p, int count) {
+  const OutsideCapture outside;
   cudaMemPool_t pool;
+  cudaStream_t stream;
   cudaError_t e = wait_for_device();
+  if (e == cudaSuccess) e = library_pool(&pool);
+  if (e == cudaSuccess) e = free_stream(&stream);
   if (e != cudaSuccess) return e;  // still in use, for all we know: not freed (as with a failing cudaFree)
-  const cudaError_t pe = library_pool(&pool);
   for (int i = 0; i < count; ++i) {
-    const cudaError_t fe = p[i] ? cudaFreeAsync(p[i], cudaStreamPerThread) : cudaSuccess;
+    const cudaError_t fe = p[i] ? cudaFreeAsync(p[i], stream) : cudaSuccess;
+    if (fe == cudaSuccess) p[i] = nullptr;
     if (e == cudaSuccess) e = fe;
   }
-  if (pe != cudaSuccess) return pe;
   uint64_t reserved = 0, used = 0;
   if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
       reserved > used + kPoolKeep) {
-    cudaStreamSynchronize(cudaStreamPerThread);
+    cudaStreamSynchronize(stream);
     cudaMemPoolTrimTo(pool, (size_t)used + kPoolKeep);
   }
   return e;
@@ -411,13 +445,15 @@ void free_stage(nabo_cuda_search* s) {
   s->stageBytes = 0;
 }
 
-void free_cloud(DeviceCloud& c) {
-  void* const p[] = {c.recs, c.nodes, c.recs32, c.coordMax};
-  object_free(p, 4);
-  c.recs = nullptr;
-  c.nodes = nullptr;
-  c.recs32 = nullptr;
-  c.coordMax = nullptr;
+// Gives an object's memory back; on an error, c still holds what was not.
+cudaError_t free_cloud(DeviceCloud& c) {
+  void* p[] = {c.recs, c.nodes, c.recs32, c.coordMax};
+  const cudaError_t e = object_free(p, 4);
+  c.recs = p[0];
+  c.nodes = p[1];
+  c.recs32 = p[2];
+  c.coordMax = static_cast<float*>(p[3]);
+  return e;
 }
 
 int create_impl(int dtype, const void* cloud, bool cloudOnDevice, int rows, int64_t n, int64_t colStride, int dimIn,
@@ -630,10 +666,12 @@ int nabo_cuda_create_device(int dtype, const void* cloud, int rows, int64_t n, i
 int nabo_cuda_destroy(nabo_cuda_search* s) {
   if (!s) return kOk;
   DeviceGuard g(s->device);
+  const OutsideCapture outside;
+  const cudaError_t e = free_cloud(s->c);
+  if (e != cudaSuccess) return cuda_error(e, "nabo_cuda_destroy");
   free_events(s);
   free_stage(s);
   destroy_pipe(s->pipe);
-  free_cloud(s->c);
   delete s;
   return kOk;
 }

@@ -45,11 +45,12 @@ cudaError_t scratch_free(void* p, cudaStream_t stream);
 // cudaFree took 35-45 us each, 150 us of a build and its destruction).
 // object_alloc is ordered on `stream`; the object's creation synchronises it
 // before anything else may use the memory. object_free waits for the device,
-// as cudaFree does (searches on any stream may still read the memory), and
-// leaves the pool with at most kPoolKeep bytes that nobody uses.
+// as cudaFree does (searches on any stream may still read the memory), nulls
+// the pointers it freed and leaves the pool with at most kPoolKeep bytes that
+// nobody uses; it may be called while any stream is being captured.
 constexpr size_t kPoolKeep = size_t(2) << 30;
 cudaError_t object_alloc(void** p, size_t bytes, cudaStream_t stream);
-cudaError_t object_free(void* const* p, int count);
+cudaError_t object_free(void** p, int count);
 // Consecutive query chunks of a pipelined search: chunk c is the queries
 // [c ? end[c-1] : 0, end[c]).
 constexpr int kMaxQueryChunks = 64;
