@@ -44,7 +44,7 @@ constexpr int kTcQueries = 128;  // per block: the accumulator's rows, one per e
 constexpr int kTcStages = 3;     // runs of tiles in shared memory
 constexpr int kTcThreads = 160;  // four epilogue warps, one that copies and multiplies
 constexpr int kTcSeedStride = 8;  // every 8th stage is read first for a starting threshold
-constexpr int kTcWaitPolls = 1 << 22;  // about a second
+constexpr int kTcDrainPolls = 1 << 26;  // for the block's own products and copies, after a wait ran out
 
 // Slots of a record of D dimensions, in whole steps of 16.
 template <int D>
@@ -129,19 +129,18 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase; false after kTcWaitPolls.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Waits for the phase; false after that many polls.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int polls) {
+  uint32_t ok;
 #pragma unroll 1
-  for (int i = 0; i < kTcWaitPolls; ++i) {
-    uint32_t ok;
+  do {
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (ok) return true;
-  }
-  return false;
+  } while (!ok && --polls > 0);
+  return ok;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -221,7 +220,9 @@ struct TcSmem {
 // k_knn_bruteforce writes them. One warp copies the tiles (operand and
 // records) and issues the products, a tile ahead of the four warps that read
 // the accumulators; thread t of those owns query t. A wait that runs out
-// leaves the pipeline, and the block's queries are then searched without it.
+// (polls) leaves the pipeline, and the block's queries are then searched
+// without it, while the products and copies already issued come to their end:
+// they read and write shared memory and accumulators that the next block gets.
 //
 // Meeting the points in cloud order, a query would insert k ln(n / k) times,
 // most of them early, with loose thresholds. So every kTcSeedStride-th tile
@@ -231,7 +232,8 @@ struct TcSmem {
 // that k points other than the query itself reach.
 template <int D, int K>
 __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
-    k_bf_tc(KnnLaunch a, const unsigned char* __restrict__ operand, TcScale s, int64_t chunk, int64_t partStride) {
+    k_bf_tc(KnnLaunch a, const unsigned char* __restrict__ operand, TcScale s, int64_t chunk, int64_t partStride,
+            int polls) {
   using S = TcSmem<D, K>;
   constexpr int kTcPoints = TcTile<K>::kPoints;
   constexpr int kSlots = TcTile<K>::kSlots;
@@ -240,9 +242,9 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
   constexpr float kSlack = 0x1p-16f * (TcShape<D>::kSlots / 16);
   constexpr int kRowGroup = TcShape<D>::kSlots / 8 * 128;
   extern __shared__ __align__(128) unsigned char tcSmem[];
-  __shared__ __align__(8) uint64_t bars[2 * kTcStages + 4];
+  __shared__ __align__(8) uint64_t bars[2 * kTcStages + 5];
   __shared__ uint32_t accBase;
-  __shared__ int failed;
+  __shared__ int failed, copiedStages, multiplied;  // copies and products issued
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* const smA = tcSmem;
   unsigned char* const smB = tcSmem + S::kA;
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
   const auto empty = [&](int i) { return smem_addr(&bars[kTcStages + i]); };
   const auto accFull = [&](int i) { return smem_addr(&bars[2 * kTcStages + i]); };
   const auto accEmpty = [&](int i) { return smem_addr(&bars[2 * kTcStages + 2 + i]); };
+  const auto drained = [&]() { return smem_addr(&bars[2 * kTcStages + 4]); };
   if (warp == 4) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&accBase)),
                  "r"(kBuffers * kTcPoints)
@@ -267,6 +270,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
       mbar_init(accFull(i), 1);
       mbar_init(accEmpty(i), 4);
     }
+    mbar_init(drained(), 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -340,7 +344,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
     }
   };
 
-  bool ok = true;
+  bool ok = polls > 0;
   if (warp == 4) {
     if (lane == 0) {
       const auto copy = [&](int g, int st) {
@@ -356,15 +360,16 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
       for (; copied < total && copied < kTcStages; ++copied) copy(copied, copied);
       int st = 0;
       uint32_t round = 0;  // uses of stage st so far, parity
+      bool product = false;
       for (int g = 0; g < total && ok; ++g) {
-        ok = mbar_wait(full(st), round);
+        ok = mbar_wait(full(st), round, polls);
         const uint64_t db = tc_descriptor(smem_addr(smB + st * S::kB), kRowGroup);
 #pragma unroll
         for (int i = 0; i < S::kTiles; ++i) {
           const int buf = (g * S::kTiles + i) % kBuffers;
           // the accumulator's previous tile has been read: use n waits for n - 1
           const int use = (g * S::kTiles + i) / kBuffers;
-          if (use > 0) ok = ok && mbar_wait(accEmpty(buf), (use - 1) & 1);
+          if (use > 0) ok = ok && mbar_wait(accEmpty(buf), (use - 1) & 1, polls);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -372,10 +377,11 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
             tc_mma(acc + buf * kTcPoints, da + k * 16, db + (i * (kTcPoints / 8) * kRowGroup) / 16 + k * 16,
                    tc_instr(kTcPoints), k > 0 ? 1u : 0u);
           tc_commit(accFull(buf));
+          product = true;
           // the stage before this one is done with once this one's second tile is due
           if (i == S::kTiles - 1 && g > 0 && copied < total) {
             const int prev = st == 0 ? kTcStages - 1 : st - 1;
-            ok = mbar_wait(empty(prev), prev < st ? round : round ^ 1);
+            ok = mbar_wait(empty(prev), prev < st ? round : round ^ 1, polls);
             if (ok) copy(copied++, prev);
           }
         }
@@ -384,12 +390,9 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
           round ^= 1;
         }
       }
-      if (!ok) {
-        failed = 1;
-        // the copies in flight land before the block may leave
-        for (int g = copied > kTcStages ? copied - kTcStages : 0; g < copied; ++g)
-          mbar_wait(full(g % kTcStages), (g / kTcStages) & 1);
-      }
+      if (!ok) failed = 1;
+      copiedStages = copied;
+      multiplied = product;
     }
     __syncwarp();
   } else {
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
 #pragma unroll 1
         for (int i = 0; i < S::kTiles; ++i) {
           const int buf = (g * S::kTiles + i) % kBuffers;
-          ok = ok && mbar_wait(accFull(buf), (g * S::kTiles + i) / kBuffers & 1);
+          ok = ok && mbar_wait(accFull(buf), (g * S::kTiles + i) / kBuffers & 1, polls);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
 #pragma unroll 1
       for (int i = 0; i < S::kTiles; ++i) {
         const int buf = (g * S::kTiles + i) % kBuffers;
-        ok = mbar_wait(accFull(buf), (g * S::kTiles + i) / kBuffers & 1);
+        ok = mbar_wait(accFull(buf), (g * S::kTiles + i) / kBuffers & 1, polls);
         if (!__all_sync(0xffffffffu, ok)) {
           ok = false;
           break;
@@ -532,7 +535,9 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
           any |= mask[part];
         }
         if (any) {
-          mbar_wait(full(st), round);  // complete: makes the copied records visible to this thread
+          // complete since before the product just read: makes the copied
+          // records visible to this thread
+          mbar_wait(full(st), round, kTcDrainPolls);
           const Rec<float, D>* const tile = smR + st * S::kStagePoints + i * kTcPoints;
           do {
             int part = 0;
@@ -566,6 +571,14 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (failed && threadIdx.x == 128) {  // the issuing thread: nothing of the block's may outlive it
+    if (multiplied) {
+      tc_commit(drained());
+      mbar_wait(drained(), 0, kTcDrainPolls);
+    }
+    for (int g = max(copiedStages - kTcStages, 0); g < copiedStages; ++g)
+      mbar_wait(full(g % kTcStages), (g / kTcStages) & 1, kTcDrainPolls);
+  }
   if (failed && warp < 4) {  // a wait ran out: this block's queries without the pipeline
     heap.init(a.k);
     cap = maxRadius2;
@@ -576,6 +589,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
       offer(r);
     }
   }
+  __syncwarp();
   if (warp == 4)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(acc), "r"(kBuffers * kTcPoints));
   if (active) {

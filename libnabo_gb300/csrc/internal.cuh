@@ -266,6 +266,9 @@ struct KnnArgs {
   // from the scratch pool.
   void* stackSlab = nullptr;
   size_t stackSlabBytes = 0;
+  // Polls after which a wait inside the tensor-core brute force gives up (about
+  // a second); tests let it run out.
+  int waitPolls = 1 << 22;
 };
 
 // Whether a search runs its queries in a sorted order. The sort costs about

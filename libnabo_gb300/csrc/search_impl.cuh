@@ -394,7 +394,7 @@ inline int64_t tc_rows(int64_t qBlocks, int64_t slots, int64_t most, int k) {
 }
 
 template <int D, int K>
-int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, cudaStream_t stream) {
+int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, int polls, cudaStream_t stream) {
   using S = TcSmem<D, K>;
   const int qBlocks = ceil_div(L.nq, kTcQueries);
   int dev = 0, sms = 152;
@@ -424,7 +424,7 @@ int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, cudaStream_t stre
     P.found = nullptr;
   }
   if (e == cudaSuccess) {
-    k_bf_tc<D, K><<<dim3(qBlocks, (unsigned)rows), kTcThreads, smem, stream>>>(P, block, s, chunk, stride);
+    k_bf_tc<D, K><<<dim3(qBlocks, (unsigned)rows), kTcThreads, smem, stream>>>(P, block, s, chunk, stride, polls);
     if (rows > 1)
       k_bf_merge<float, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(P.outIdx, static_cast<const float*>(P.outD2),
                                                                     (int)rows, stride, L.nq, L.k, L.outIdx,
@@ -453,7 +453,7 @@ int knn_bruteforce(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream) 
     if (!done && c.n >= 512 && tc_scale(c, &s)) {
 #define NABO_LAUNCH(KK)                                   \
   case KK:                                                \
-    rc = launch_bruteforce_tc<D, KK>(L, s, stream);       \
+    rc = launch_bruteforce_tc<D, KK>(L, s, a.waitPolls, stream); \
     break;
       switch (K) { NABO_K_LIST(NABO_LAUNCH) }
 #undef NABO_LAUNCH
