@@ -1208,6 +1208,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
     ta.bucket = bucket;
     ta.maxLevels = maxLevels;
     ta.smallCap = (int)smallCap;
+    ta.barrierPolls = f->barrierPolls;
     ta.workBytes = (int64_t)withLists;
     const void* kernel = topMode == kTopResident ? (const void*)k_top<T, D, kTopResident>
                          : topMode == kTopLists  ? (const void*)k_top<T, D, kTopLists>

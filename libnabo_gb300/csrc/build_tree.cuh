@@ -162,7 +162,6 @@ __device__ __forceinline__ T coord_of(const Rec<T, D>& r, int cd) {
 constexpr int kTopThreads = 1024;
 constexpr int kTopWarps = kTopThreads / 32;
 constexpr int kTopMinChunk = 1024;
-constexpr int kTopSpinLimit = 1 << 22;
 constexpr size_t kTopSmemMax = 200 * 1024;
 
 template <typename T, int D>
@@ -204,7 +203,7 @@ struct TopArgs {
   TopState* st;
   int* counters;
   const int* nonFinite;  // stop at once if set (null: never)
-  int n, nClouds, dim, chunk, pieces, smallMax, bucket, maxLevels, smallCap;
+  int n, nClouds, dim, chunk, pieces, smallMax, bucket, maxLevels, smallCap, barrierPolls;
 };
 
 // A block's working memory: the chunk's records (when resident), two lists of
@@ -223,18 +222,29 @@ struct TopShape {
 };
 
 // Waits until every block has arrived as often as this one (all blocks are
-// resident: cooperative launch). False after kTopSpinLimit polls.
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target) {
+// resident: cooperative launch). False after that many polls, and then in
+// every block: one that gives up takes its arrival back, unless all have
+// arrived by then, so that no other passes. The blocks then leave one after
+// another, every record still in one place, and the build reports that it did
+// not finish.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, int polls) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(count, 1u);
     int good = 0;
-    for (int i = 0; i < kTopSpinLimit && !good; ++i) {
+    for (int i = 0; i < polls && !good; ++i) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
       good = (int)(v - target) >= 0;
+    }
+    if (!good) {
+      for (unsigned v = atomicAdd(count, 0u); !(good = (int)(v - target) >= 0);) {
+        const unsigned old = atomicCAS(count, v, v - 1u);
+        if (old == v) break;
+        v = old;
+      }
     }
     __threadfence();
     ok = good;
@@ -325,7 +335,7 @@ __global__ void __launch_bounds__(kTopThreads, 1) k_top(const TopArgs<T, D> a) {
   unsigned arrive = 0;
   const auto barrier = [&]() {
     arrive += gridDim.x;
-    if (grid_barrier(&a.st->barrier, arrive)) return true;
+    if (grid_barrier(&a.st->barrier, arrive, a.barrierPolls)) return true;
     if (threadIdx.x == 0) atomicOr(a.counters + kFlags, 1);
     return false;
   };

@@ -131,6 +131,9 @@ struct ForestOut {
   void* rootLo = nullptr;
   void* rootHi = nullptr;
   int* status = nullptr;
+  // Polls after which a wait between the blocks of the top levels gives up
+  // (some seconds); tests let it run out.
+  int barrierPolls = 1 << 22;
 };
 
 // A batched search over a forest (batch.cu).

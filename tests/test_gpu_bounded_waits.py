@@ -1,5 +1,6 @@
 """Waits inside kernels have a limit. When one runs out, a brute-force block searches its queries without the pipeline and
-leaves nothing of it behind (tests/cpp/brute_force_waits.cu, over the library's internal entry points)."""
+leaves nothing of it behind; a tree build reports that it did not finish (tests/cpp/*_waits.cu, over the library's
+internal entry points)."""
 import os
 import subprocess
 
@@ -24,3 +25,8 @@ def compile_cu(tmp_path, name):
 def test_brute_force_waits_that_run_out(tmp_path):
     r = subprocess.run([compile_cu(tmp_path, "brute_force_waits")], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.count("ok ") == 5, r.stdout + r.stderr
+
+
+def test_build_waits_that_run_out(tmp_path):
+    r = subprocess.run([compile_cu(tmp_path, "build_waits")], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.count("ok ") == 3, r.stdout + r.stderr
