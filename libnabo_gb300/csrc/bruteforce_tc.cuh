@@ -36,6 +36,7 @@
 
 #include <cuda_fp16.h>
 
+#include "internal.cuh"
 #include "search.cuh"
 
 namespace nabo_gb300 {
@@ -53,13 +54,6 @@ struct TcShape {
   static constexpr int kSteps = kSlots / 16;
   static constexpr int kRowBytes = kSlots * 2;
   static constexpr size_t operandBytes(int rows) { return (size_t)rows * kRowBytes; }
-};
-
-struct TcScale {
-  float centre[kMaxDim];
-  float scale;    // s, a power of 2
-  float scale2;   // s^2
-  float pointMax; // P
 };
 
 // Shared-memory operand layout (K-major, no swizzle): 8 rows by 16 bytes are
@@ -101,7 +95,9 @@ __device__ __forceinline__ void tc_row(const float (&x)[D], Put&& put) {
   }
 }
 
-// The points' operand, padded to whole tiles (the padding is never tested).
+// The points' operand, padded to whole tiles (the padding is never tested). It
+// depends on the cloud only, so an object holds it from its creation and a
+// search needs no scratch for it.
 template <int D>
 __global__ void k_bf_tc_points(const Rec<float, D>* __restrict__ recs, int64_t n, int64_t padded, int dim, TcScale s,
                                unsigned char* out) {

@@ -67,6 +67,12 @@ thread_local bool g_captureAllocations = false;
 
 void set_capture_allocations(bool on) { g_captureAllocations = on; }
 
+bool caller_captures(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (!g_captureAllocations && cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+  return status != cudaStreamCaptureStatusNone;
+}
+
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t stream) {
   // while a CUDA graph is being captured, allocations become graph memory
   // nodes of the device's default pool
@@ -407,7 +413,11 @@ int build_any(nabo_cuda_search* h, const void* dCloud, int64_t stride, cudaStrea
     if (rc == kOk && h->c.dtype == NABO_CUDA_FLOAT64) rc = narrow_cloud(h->c, st);
     return rc;
   }
-  NABO_DISPATCH(h->c.dtype, h->c.dpad, (pack_cloud<T, D>(static_cast<const T*>(dCloud), h->c.n, stride, h->c.dim, st, &h->c)));
+  int rc = kOk;
+  NABO_DISPATCH_RC(rc, h->c.dtype, h->c.dpad,
+                   (pack_cloud<T, D>(static_cast<const T*>(dCloud), h->c.n, stride, h->c.dim, st, &h->c)));
+  if (rc == kOk) NABO_DISPATCH_RC(rc, h->c.dtype, h->c.dpad, (prepare_bruteforce<T, D>(h->c, st)));
+  return rc;
 }
 
 int knn_any(const nabo_cuda_search* h, const KnnArgs& a, cudaStream_t st) {
@@ -447,12 +457,13 @@ void free_stage(nabo_cuda_search* s) {
 
 // Gives an object's memory back; on an error, c still holds what was not.
 cudaError_t free_cloud(DeviceCloud& c) {
-  void* p[] = {c.recs, c.nodes, c.recs32, c.coordMax};
-  const cudaError_t e = object_free(p, 4);
+  void* p[] = {c.recs, c.nodes, c.recs32, c.coordMax, c.tcOperand};
+  const cudaError_t e = object_free(p, 5);
   c.recs = p[0];
   c.nodes = p[1];
   c.recs32 = p[2];
   c.coordMax = static_cast<float*>(p[3]);
+  c.tcOperand = p[4];
   return e;
 }
 

@@ -83,6 +83,17 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 // While set (calling thread only), scratch_alloc uses cudaMallocAsync so the
 // allocations can be captured into a CUDA graph.
 void set_capture_allocations(bool on);
+// Whether a caller (not the library itself) is capturing the stream.
+bool caller_captures(cudaStream_t stream);
+
+// Coordinates of the tensor-core brute force (bruteforce_tc.cuh): s (x - c),
+// with P at least every point's squared norm.
+struct TcScale {
+  float centre[kMaxDim];
+  float scale;    // s, a power of 2
+  float scale2;   // s^2
+  float pointMax; // P
+};
 
 // Device-resident kd-tree (or, for brute force, the packed cloud only).
 struct DeviceCloud {
@@ -102,6 +113,10 @@ struct DeviceCloud {
   // coordinate magnitude (device float), for the search's float pre-filter
   void* recs32 = nullptr;
   float* coordMax = nullptr;
+  // float brute force: the points as the tensor cores' operand and its
+  // coordinates (prepare_bruteforce), or null
+  void* tcOperand = nullptr;
+  TcScale tc = {};
 };
 
 struct BuildStats {
@@ -288,6 +303,10 @@ template <typename T, int D>
 int knn_kdtree(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream);
 template <typename T, int D>
 int knn_bruteforce(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream);
+// After pack_cloud: what else the brute-force search keeps of the cloud. An
+// object for which there is no room searches without it.
+template <typename T, int D>
+int prepare_bruteforce(DeviceCloud& c, cudaStream_t stream);
 
 template <typename T, int D>
 int knn_kdtree_given_order(const DeviceCloud& c, const KnnArgs& a, const int32_t* order, cudaStream_t stream);

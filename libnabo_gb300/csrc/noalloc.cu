@@ -284,7 +284,7 @@ extern "C" int nabo_cuda_knn_device_noalloc(const nabo_cuda_search* s, const voi
     }
   } else {
     rc = set_error(kErrArgument, "nabo_cuda_knn_device_noalloc serves kd-tree objects; "
-                                 "the brute-force search needs no scratch (nabo_cuda_knn_device runs without when it can get none)");
+                                 "nabo_cuda_knn_device searches brute-force objects, with at most scratch that it can do without");
   }
   if (prev >= 0 && prev != h.device) cudaSetDevice(prev);
   return rc;

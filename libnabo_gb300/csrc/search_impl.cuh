@@ -141,6 +141,12 @@ int launch_wide_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
   return k_unsupported();
 }
 
+inline int sm_count() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Queries per warp of the one-thread-per-query search. A warp takes as long as
 // its lanes' paths together where they diverge, so a search too small to fill
 // the GPU runs fewer queries in each of more warps: the fewest lanes (a power
@@ -151,8 +157,7 @@ int launch_wide_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
 // 60; 30 k: 99, 93, 105, 136, ...; 83 k: 116, 138, 175, ...: past 16 warps
 // per SM the extra warps only repeat instructions.
 inline int spread_lanes(int64_t nq) {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   int lanes = 1;
   while (lanes < 32 && nq > (int64_t)lanes * 16 * sms) lanes *= 2;
   return lanes;
@@ -314,38 +319,56 @@ int knn_kdtree(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream) {
 // 4.79 -> 5.78 ms at k = 10: each row's top-k lists start empty, and more
 // of the points then meet a loose threshold.)
 constexpr int kBfBlocksPerSm = 8;
+template <typename T, int D>
+constexpr int64_t kBfTile = (int64_t)((24 * 1024) / sizeof(Rec<T, D>));
+template <typename T, int D, int QT>
+int64_t bf_rows(int64_t n, int64_t nq) {
+  const int qBlocks = ceil_div(nq, 128 * QT);
+  const int64_t tiles = std::max<int64_t>(1, (n + kBfTile<T, D> - 1) / kBfTile<T, D>);
+  return std::min<int64_t>({(kBfBlocksPerSm * (int64_t)sm_count() + qBlocks - 1) / qBlocks, tiles / 4, 64});
+}
+
+// The block rows' lists, k per query and row, from one scratch block; none
+// (and one row) when it cannot be had.
+struct RowLists {
+  unsigned char* block = nullptr;
+  size_t idxBytes = 0;
+  RowLists(int64_t entries, size_t distBytes, cudaStream_t stream) {
+    idxBytes = ((size_t)entries * sizeof(int32_t) + 255) / 256 * 256;
+    if (scratch_alloc((void**)&block, idxBytes + (size_t)entries * distBytes, stream) != cudaSuccess) {
+      cudaGetLastError();
+      block = nullptr;
+    }
+  }
+  int32_t* idx() const { return reinterpret_cast<int32_t*>(block); }
+  void* d2() const { return block + idxBytes; }
+};
+
 template <typename T, int D, int K, int QT = BfShape<T, K>::QT, int J = BfShape<T, K>::J>
 int launch_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
-  constexpr int64_t kTile = (int64_t)((24 * 1024) / sizeof(Rec<T, D>));
+  constexpr int64_t kTile = kBfTile<T, D>;
   const int qBlocks = ceil_div(L.nq, 128 * QT);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t tiles = std::max<int64_t>(1, (L.n + kTile - 1) / kTile);
-  int64_t rows = std::min<int64_t>({(kBfBlocksPerSm * (int64_t)sms + qBlocks - 1) / qBlocks, tiles / 4, 64});
-  if (rows <= 1) {
-    k_knn_bruteforce<T, D, K, QT, J><<<qBlocks, 128, 0, stream>>>(L, L.n, 0);
-    return kOk;
+  int64_t rows = bf_rows<T, D, QT>(L.n, L.nq);
+  if (rows > 1) {
+    const int64_t tiles = (L.n + kTile - 1) / kTile;
+    const int64_t chunk = (tiles + rows - 1) / rows * kTile;
+    rows = (L.n + chunk - 1) / chunk;
+    const int64_t stride = L.nq * (int64_t)L.k;
+    const RowLists lists(rows * stride, sizeof(T), stream);
+    if (lists.block) {
+      KnnLaunch P = L;
+      P.outIdx = lists.idx();
+      P.outD2 = lists.d2();
+      P.found = nullptr;
+      k_knn_bruteforce<T, D, K, QT, J><<<dim3(qBlocks, (unsigned)rows), 128, 0, stream>>>(P, chunk, stride);
+      k_bf_merge<T, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(lists.idx(), static_cast<const T*>(lists.d2()), (int)rows,
+                                                               stride, L.nq, L.k, L.outIdx, static_cast<T*>(L.outD2),
+                                                               L.found);
+      scratch_free(lists.block, stream);
+      return kOk;
+    }
   }
-  const int64_t chunk = (tiles + rows - 1) / rows * kTile;
-  rows = (L.n + chunk - 1) / chunk;
-  const int64_t stride = L.nq * (int64_t)L.k;
-  int32_t* pIdx = nullptr;
-  T* pD2 = nullptr;
-  NABO_CUDA_TRY(scratch_alloc((void**)&pIdx, (size_t)(rows * stride) * sizeof(int32_t), stream));
-  cudaError_t e = scratch_alloc((void**)&pD2, (size_t)(rows * stride) * sizeof(T), stream);
-  if (e != cudaSuccess) {
-    scratch_free(pIdx, stream);
-    return cuda_error(e, "brute-force partial results");
-  }
-  KnnLaunch P = L;
-  P.outIdx = pIdx;
-  P.outD2 = pD2;
-  P.found = nullptr;
-  k_knn_bruteforce<T, D, K, QT, J><<<dim3(qBlocks, (unsigned)rows), 128, 0, stream>>>(P, chunk, stride);
-  k_bf_merge<T, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(pIdx, pD2, (int)rows, stride, L.nq, L.k, L.outIdx,
-                                                           static_cast<T*>(L.outD2), L.found);
-  scratch_free(pIdx, stream);
-  scratch_free(pD2, stream);
+  k_knn_bruteforce<T, D, K, QT, J><<<qBlocks, 128, 0, stream>>>(L, L.n, 0);
   return kOk;
 }
 
@@ -393,46 +416,64 @@ inline int64_t tc_rows(int64_t qBlocks, int64_t slots, int64_t most, int k) {
   return best;
 }
 
+// The search over an object's operand. Its only scratch is the lists of block
+// rows. A call that a caller captures takes rows only where k_knn_bruteforce
+// would: memory nodes would keep the graph from being instantiated twice or
+// used inside another one.
 template <int D, int K>
-int launch_bruteforce_tc(const KnnLaunch& L, const TcScale& s, int polls, cudaStream_t stream) {
+int launch_bruteforce_tc(const KnnLaunch& L, const DeviceCloud& c, int polls, cudaStream_t stream) {
   using S = TcSmem<D, K>;
   const int qBlocks = ceil_div(L.nq, kTcQueries);
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t stages = (L.n + S::kStagePoints - 1) / S::kStagePoints;
   const int perSm = std::min(TcTile<K>::kBlocksPerSm, 228 * 1024 / (S::kRequest + 1024));
-  int64_t rows = tc_rows(qBlocks, (int64_t)perSm * sms, std::min<int64_t>(stages / kTcSeedStride, 64), L.k);
-  const int64_t chunk = (stages + rows - 1) / rows * S::kStagePoints;
-  rows = (L.n + chunk - 1) / chunk;
-  const int64_t padded = stages * S::kStagePoints;
-  const int64_t stride = rows > 1 ? L.nq * (int64_t)L.k : 0;
-  const size_t operandBytes = TcShape<D>::operandBytes(1) * (size_t)padded;
-  const size_t idxBytes = ((size_t)(rows * stride) * sizeof(int32_t) + 255) / 256 * 256;
-  unsigned char* block = nullptr;  // operand | partial indices | partial distances
-  if (scratch_alloc((void**)&block, operandBytes + 2 * idxBytes, stream) != cudaSuccess) {
-    cudaGetLastError();  // no room for the operand: the kernel that needs none
-    return launch_bruteforce<float, D, K>(L, stream);
-  }
-  k_bf_tc_points<D><<<ceil_div(padded, 256), 256, 0, stream>>>(static_cast<const Rec<float, D>*>(L.recs), L.n, padded,
-                                                               L.dim, s, block);
+  int64_t rows = tc_rows(qBlocks, (int64_t)perSm * sm_count(), std::min<int64_t>(stages / kTcSeedStride, 64), L.k);
+  if (rows > 1 && bf_rows<float, D, BfShape<float, K>::QT>(L.n, L.nq) <= 1 && caller_captures(stream)) rows = 1;
   constexpr int smem = S::kRequest;
-  cudaError_t e = cudaFuncSetAttribute(k_bf_tc<D, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  KnnLaunch P = L;
+  NABO_CUDA_TRY(cudaFuncSetAttribute(k_bf_tc<D, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const unsigned char* operand = static_cast<const unsigned char*>(c.tcOperand);
   if (rows > 1) {
-    P.outIdx = reinterpret_cast<int32_t*>(block + operandBytes);
-    P.outD2 = block + operandBytes + idxBytes;
-    P.found = nullptr;
+    const int64_t chunk = (stages + rows - 1) / rows * S::kStagePoints;
+    rows = (L.n + chunk - 1) / chunk;
+    const int64_t stride = L.nq * (int64_t)L.k;
+    const RowLists lists(rows * stride, sizeof(float), stream);
+    if (lists.block) {
+      KnnLaunch P = L;
+      P.outIdx = lists.idx();
+      P.outD2 = lists.d2();
+      P.found = nullptr;
+      k_bf_tc<D, K><<<dim3(qBlocks, (unsigned)rows), kTcThreads, smem, stream>>>(P, operand, c.tc, chunk, stride, polls);
+      k_bf_merge<float, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(lists.idx(), static_cast<const float*>(lists.d2()),
+                                                                   (int)rows, stride, L.nq, L.k, L.outIdx,
+                                                                   static_cast<float*>(L.outD2), L.found);
+      scratch_free(lists.block, stream);
+      return kOk;
+    }
   }
-  if (e == cudaSuccess) {
-    k_bf_tc<D, K><<<dim3(qBlocks, (unsigned)rows), kTcThreads, smem, stream>>>(P, block, s, chunk, stride, polls);
-    if (rows > 1)
-      k_bf_merge<float, K><<<ceil_div(L.nq, 128), 128, 0, stream>>>(P.outIdx, static_cast<const float*>(P.outD2),
-                                                                    (int)rows, stride, L.nq, L.k, L.outIdx,
-                                                                    static_cast<float*>(L.outD2), L.found);
-    e = cudaGetLastError();
+  k_bf_tc<D, K><<<qBlocks, kTcThreads, smem, stream>>>(L, operand, c.tc, stages * S::kStagePoints, 0, polls);
+  return kOk;
+}
+
+// (us, without / with the tensor cores: 64 points, 100 k queries 35 / 59; 256
+// points 90 / 93; 500 points, 5 k queries 59 / 48; 100 k points, one query
+// 176 / 71)
+constexpr int64_t kTcMinPoints = 512;
+
+template <typename T, int D>
+int prepare_bruteforce(DeviceCloud& c, cudaStream_t stream) {
+  if constexpr (sizeof(T) == 4) {
+    if (c.n < kTcMinPoints || !tc_scale(c, &c.tc)) return kOk;
+    constexpr int kStage = TcSmem<D, 1>::kStagePoints;
+    const int64_t padded = (c.n + kStage - 1) / kStage * kStage;
+    if (object_alloc(&c.tcOperand, TcShape<D>::operandBytes(1) * (size_t)padded, stream) != cudaSuccess) {
+      cudaGetLastError();
+      c.tcOperand = nullptr;
+      return kOk;
+    }
+    k_bf_tc_points<D><<<ceil_div(padded, 256), 256, 0, stream>>>(static_cast<const Rec<float, D>*>(c.recs), c.n, padded,
+                                                                 c.dim, c.tc, static_cast<unsigned char*>(c.tcOperand));
+    NABO_CUDA_TRY(cudaGetLastError());
   }
-  scratch_free(block, stream);
-  return e == cudaSuccess ? kOk : cuda_error(e, "tensor-core brute force");
+  return kOk;
 }
 
 template <typename T, int D>
@@ -446,14 +487,10 @@ int knn_bruteforce(const DeviceCloud& c, const KnnArgs& a, cudaStream_t stream) 
   if (K < 0) rc = launch_wide_bruteforce<T, D>(L, stream);
   bool done = K < 0;
   if constexpr (sizeof(T) == 4) {
-    TcScale s;
-    // (us, without / with the tensor cores: 64 points, 100 k queries 35 / 59;
-    // 256 points 90 / 93; 500 points, 5 k queries 59 / 48; 100 k points, one
-    // query 176 / 71)
-    if (!done && c.n >= 512 && tc_scale(c, &s)) {
-#define NABO_LAUNCH(KK)                                   \
-  case KK:                                                \
-    rc = launch_bruteforce_tc<D, KK>(L, s, a.waitPolls, stream); \
+    if (!done && c.tcOperand) {
+#define NABO_LAUNCH(KK)                                          \
+  case KK:                                                       \
+    rc = launch_bruteforce_tc<D, KK>(L, c, a.waitPolls, stream); \
     break;
       switch (K) { NABO_K_LIST(NABO_LAUNCH) }
 #undef NABO_LAUNCH
@@ -684,6 +721,7 @@ int knn_batch(const BatchArgs& b, cudaStream_t stream) {
   template int knn_leaf_order<T, D>(const DeviceCloud&, const void*, int64_t, int64_t, int32_t*, cudaStream_t); \
   template int knn_kdtree<T, D>(const DeviceCloud&, const KnnArgs&, cudaStream_t); \
   template int knn_bruteforce<T, D>(const DeviceCloud&, const KnnArgs&, cudaStream_t); \
+  template int prepare_bruteforce<T, D>(DeviceCloud&, cudaStream_t);               \
   template int knn_kdtree_given_order<T, D>(const DeviceCloud&, const KnnArgs&, const int32_t*, cudaStream_t); \
   template int knn_chunk_order<T, D>(const DeviceCloud&, const void*, int64_t, int64_t, const QueryChunks&, int32_t*, \
                                      cudaStream_t, void*);
