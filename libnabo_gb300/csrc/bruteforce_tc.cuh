@@ -12,17 +12,17 @@
 // so results are those of k_knn_bruteforce, bit for bit.
 //
 // Bound by the ALU pipe (64 % busy: the minimum, the tests, the waits' polls)
-// and the exact tests. Kernel ms, k_knn_bruteforce -> here: 100 k x 100 k 3-D
-// points, k = 1 2.80 -> 1.13, 5 3.51 -> 1.54, 10 4.81 -> 2.10, 16 7.13 -> 2.47,
-// 32 17.3 -> 4.30; 50 k points, 40 k queries in 8-D, k = 5 1.90 -> 0.55; 30 k x
-// 30 k in 16-D, k = 10 2.71 -> 0.45; 100 k points, one query 0.18 -> 0.07.
+// and the exact tests. A search's ms, k_knn_bruteforce -> here: 100 k x 100 k
+// 3-D points, k = 1 2.80 -> 1.15, 5 3.51 -> 1.54, 10 4.81 -> 2.00, 16 7.13 ->
+// 2.17, 32 17.3 -> 3.56; 50 k points, 40 k queries in 8-D, k = 5 1.90 -> 0.51;
+// 30 k x 30 k in 16-D, k = 10 2.71 -> 0.43; 100 k points, one query 0.18 -> 0.08.
 //
-// Coordinates enter as x' = s (x - c), c the cloud's box centre and s the
-// power of 2 that brings the box to at most 1 from it, each as h + l with h
-// and l fp16: |x' - h - l| <= 2^-22 |x'| + 2^-25. Per dimension the product
-// takes three slots, (-2 qh) ph + (-2 ql) ph + (-2 qh) pl, and |p'|^2 two more
-// against ones. With X = |q'|^2 + P, P >= |p'|^2 for every point (P >= 1/4),
-// the value's error is at most
+// Coordinates enter as x' = s (x - c), with c and the power of 2 s from a
+// sample of the points (tc_scale: all but a few of them within 8 of c), each
+// as h + l with h and l fp16: |x' - h - l| <= 2^-22 |x'| + 2^-25. Per
+// dimension the product takes three slots, (-2 qh) ph + (-2 ql) ph + (-2 qh)
+// pl, and |p'|^2 two more against ones. With X = |q'|^2 + P, P >= |p'|^2 for
+// the points of a stage (P >= 1/4), the value's error is at most
 //   2^-22 X          the dropped ql pl,
 //   2^-20 X          the split's and the centring's rounding (the fp16
 //                    subnormals' 2^-25 included, P being at least 1/4),
@@ -32,6 +32,18 @@
 // the exact scaled distance for D <= 16. The threshold's slack is
 // 2^-16 (S / 16) (s^2 thr + 2 X): over twice the sum for every S from 16 on.
 // (Measured against 64 bits over 2-D to 16-D points: at most 2^-21.3 X.)
+//
+// The slack grows with P, so P is a stage's own, and a point farther out than
+// nearly all the others (|p'|^2 above TcShape::kFar) leaves it: its value is
+// minus infinity, below every threshold, so that every query takes its exact
+// distance. One far return among a scan's points costs each query one distance
+// (with one centre, scale and P for the whole cloud most points passed every
+// threshold). A query that the filter cannot hold is searched after the others,
+// by its warp without the pipeline.
+// (82,762 lidar points and as many queries, k = 5, ms, k_knn_bruteforce / one
+// range for the whole cloud / here: the scan 6.39 / 3.95 / 3.05, one return at
+// 10 km 6.54 / 17.85 / 3.10, 2 % at 1 km 7.40 / 12.89 / 3.6; 80 k points of a
+// Cauchy law 7.46 / 15.25 / 2.73, log-normal 7.45 / 14.85 / 5.54.)
 #pragma once
 
 #include <cuda_fp16.h>
@@ -45,6 +57,7 @@ constexpr int kTcQueries = 128;  // per block: the accumulator's rows, one per e
 constexpr int kTcStages = 3;     // runs of tiles in shared memory
 constexpr int kTcThreads = 160;  // four epilogue warps, one that copies and multiplies
 constexpr int kTcSeedStride = 8;  // every 8th stage is read first for a starting threshold
+constexpr float kTcQueryMax = 32736.0f;  // largest |x'| of a query that the filter holds (-2 x' is an fp16)
 constexpr int kTcDrainPolls = 1 << 26;  // for the block's own products and copies, after a wait ran out
 
 // Slots of a record of D dimensions, in whole steps of 16.
@@ -52,8 +65,18 @@ template <int D>
 struct TcShape {
   static constexpr int kSlots = (3 * D + 2 + 15) / 16 * 16;
   static constexpr int kSteps = kSlots / 16;
+  static constexpr float kFar = 128.0f * D;  // all coordinates within 11 of the centre are below
   static constexpr int kRowBytes = kSlots * 2;
   static constexpr size_t operandBytes(int rows) { return (size_t)rows * kRowBytes; }
+};
+
+// Points copied at a time: several tiles, so that the copying thread's work
+// per tile stays below what the multiplying needs. Their operand is followed
+// by their P in 16 bytes, its sign set when some of them are far.
+template <int D>
+struct TcStage {
+  static constexpr int kPoints = D <= 4 ? 256 : 128;
+  static constexpr int kBytes = (int)TcShape<D>::operandBytes(kPoints) + 16;
 };
 
 // Shared-memory operand layout (K-major, no swizzle): 8 rows by 16 bytes are
@@ -65,9 +88,9 @@ __host__ __device__ __forceinline__ int64_t tc_offset(int64_t row, int slot8) {
 }
 
 // Writes one row of an operand, its 16-byte blocks through `put(block, uint4)`.
-// Queries: -2 q'; points: p' and |p'|^2.
+// Queries: -2 q'; points: p' and |p'|^2 (a far point, x = 0: minus infinity).
 template <int D, bool QUERY, typename Put>
-__device__ __forceinline__ void tc_row(const float (&x)[D], Put&& put) {
+__device__ __forceinline__ void tc_row(const float (&x)[D], bool far, Put&& put) {
   __half slot[TcShape<D>::kSlots];
 #pragma unroll
   for (int i = 0; i < TcShape<D>::kSlots; ++i) slot[i] = __float2half(0.0f);
@@ -83,7 +106,7 @@ __device__ __forceinline__ void tc_row(const float (&x)[D], Put&& put) {
     n2 = fmaf(x[d], x[d], n2);
   }
   const __half nh = __float2half_rn(n2);
-  slot[3 * D] = QUERY ? __float2half(1.0f) : nh;
+  slot[3 * D] = QUERY ? __float2half(1.0f) : (far ? __ushort_as_half(0xfc00u) : nh);
   slot[3 * D + 1] = QUERY ? __float2half(1.0f) : __float2half_rn(n2 - __half2float(nh));
 #pragma unroll
   for (int b = 0; b < TcShape<D>::kSlots / 8; ++b) {
@@ -95,14 +118,16 @@ __device__ __forceinline__ void tc_row(const float (&x)[D], Put&& put) {
   }
 }
 
-// The points' operand, padded to whole tiles (the padding is never tested). It
-// depends on the cloud only, so an object holds it from its creation and a
-// search needs no scratch for it.
+// The points' operand, a block per stage, padded to whole stages (the padding
+// is never tested). It depends on the cloud only, so an object holds it from
+// its creation and a search needs no scratch for it.
 template <int D>
-__global__ void k_bf_tc_points(const Rec<float, D>* __restrict__ recs, int64_t n, int64_t padded, int dim, TcScale s,
-                               unsigned char* out) {
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= padded) return;
+__global__ void __launch_bounds__(TcStage<D>::kPoints)
+    k_bf_tc_points(const Rec<float, D>* __restrict__ recs, int64_t n, int dim, TcScale s, unsigned char* out) {
+  __shared__ unsigned largest;  // a non-negative float's bits order like its value
+  if (threadIdx.x == 0) largest = 0u;
+  const int64_t p = blockIdx.x * (int64_t)TcStage<D>::kPoints + threadIdx.x;
+  unsigned char* const stage = out + blockIdx.x * (int64_t)TcStage<D>::kBytes;
   float x[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) x[d] = 0.0f;
@@ -112,7 +137,23 @@ __global__ void k_bf_tc_points(const Rec<float, D>* __restrict__ recs, int64_t n
 #pragma unroll
     for (int d = 0; d < D; ++d) x[d] = d < dim ? (r.p.c[d] - s.centre[d]) * s.scale : 0.0f;
   }
-  tc_row<D, false>(x, [&](int b, uint4 v) { *reinterpret_cast<uint4*>(out + tc_offset<D>(p, b)) = v; });
+  float n2 = 0.0f;
+#pragma unroll
+  for (int d = 0; d < D; ++d) n2 = fmaf(x[d], x[d], n2);
+  const bool far = !(n2 <= TcShape<D>::kFar);
+#pragma unroll
+  for (int d = 0; d < D; ++d) x[d] = far ? 0.0f : x[d];
+  tc_row<D, false>(x, far, [&](int b, uint4 v) {
+    *reinterpret_cast<uint4*>(stage + tc_offset<D>(threadIdx.x, b)) = v;
+  });
+  const int anyFar = __syncthreads_or(far);
+  const unsigned most = __reduce_max_sync(0xffffffffu, __float_as_uint(far ? 0.0f : n2));
+  if ((threadIdx.x & 31) == 0) atomicMax(&largest, most);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const float P = fmaxf(0.25f, __uint_as_float(largest) * (1.0f + 1e-5f));
+    *reinterpret_cast<float4*>(stage + TcStage<D>::kBytes - 16) = make_float4(anyFar ? -P : P, 0.0f, 0.0f, 0.0f);
+  }
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -198,12 +239,11 @@ struct TcTile {
 
 template <int D, int K>
 struct TcSmem {
-  // points copied at a time: several tiles, so that the copying thread's work
-  // per tile stays below what the multiplying needs
-  static constexpr int kStagePoints = D <= 4 ? 256 : 128;
+  static constexpr int kStagePoints = TcStage<D>::kPoints;
   static constexpr int kTiles = kStagePoints / TcTile<K>::kPoints;
   static constexpr int kA = (int)TcShape<D>::operandBytes(kTcQueries);
-  static constexpr int kB = (int)TcShape<D>::operandBytes(kStagePoints);
+  static constexpr int kCopy = TcStage<D>::kBytes;
+  static constexpr int kB = (kCopy + 127) / 128 * 128;
   static constexpr int kRecs = kStagePoints * (int)sizeof(Rec<float, D>);
   static constexpr int kBytes = kA + kTcStages * (kB + kRecs);
   // enough that no more blocks share an SM than its accumulators allow
@@ -223,8 +263,8 @@ struct TcSmem {
 // Meeting the points in cloud order, a query would insert k ln(n / k) times,
 // most of them early, with loose thresholds. So every kTcSeedStride-th tile
 // is read once before, only for a starting threshold: the smallest filter
-// value of each of kSlots groups of its points. The (k + 1)-th smallest of
-// those, brought back to a distance with the filter's slack, is a distance
+// value of each of kSlots groups of its points (far ones left out). The
+// (k + 1)-th smallest of those, brought back to a distance with the filter's slack, is a distance
 // that k points other than the query itself reach.
 template <int D, int K>
 __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
@@ -276,18 +316,17 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
   float q[D];
   float maxRadius2 = __builtin_nanf("");  // an idle slot wants nothing
   float qn = 0.0f;
-  bool always = false;  // the filter cannot hold this query: every point is tested
+  bool beyond = false;  // the filter cannot hold this query
   TopK<float, K> heap;
   heap.init(a.k);
   if (warp < 4) {
     float x[D];
-    float big = 0.0f;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       q[d] = active && d < a.dim ? static_cast<const float*>(a.query)[qi * a.qStride + d] : 0.0f;
       x[d] = d < a.dim ? (q[d] - s.centre[d]) * s.scale : 0.0f;
-      big = fmaxf(big, fabsf(x[d]));
-      always = always || !(fabsf(x[d]) <= 1024.0f);
+      qn = fmaf(x[d], x[d], qn);
+      beyond = beyond || !(fabsf(x[d]) <= kTcQueryMax);
     }
     if (active) {
       maxRadius2 = (float)a.maxRadius2;
@@ -297,11 +336,9 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
       }
     }
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (!active || always) x[d] = 0.0f;
-      qn = fmaf(x[d], x[d], qn);
-    }
-    tc_row<D, true>(x, [&](int b, uint4 v) {
+    for (int d = 0; d < D; ++d) x[d] = beyond ? 0.0f : x[d];
+    qn = beyond ? 0.0f : qn;
+    tc_row<D, true>(x, false, [&](int b, uint4 v) {
       *reinterpret_cast<uint4*>(smA + tc_offset<D>(threadIdx.x, b)) = v;
     });
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -320,17 +357,17 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
     return first + (int64_t)(g < seeds ? g * kTcSeedStride : g - seeds) * S::kStagePoints;
   };
 
-  float cap = maxRadius2;  // the radius, and the seed's threshold
+  // the radius, and the seed's threshold
+  float cap = beyond ? __int_as_float(0x7fffffff) : maxRadius2;
   float thr = bf_threshold(heap.head(), cap);
-  float thrA;
-  // A NaN threshold (an idle slot, a NaN radius) passes nothing; an infinite
-  // or overflowing one passes everything to the exact test.
-  const auto set_threshold = [&]() {
-    const float t = thr * s.scale2;
-    thrA = thr != thr ? -__int_as_float(0x7f800000)
-                      : (always ? __int_as_float(0x7f800000) : (t - qn) + kSlack * (t + 2.0f * (s.pointMax + qn)));
-  };
-  set_threshold();
+  // The threshold on the filter's values, s^2 thr - |q'|^2 with the slack for
+  // this stage's P: one multiply-add from a query's part and the stage's. A
+  // NaN threshold (an idle slot, a NaN radius, a query beyond the filter)
+  // passes nothing; an infinite or overflowing one passes everything to the
+  // exact test.
+  const float queryPart = (2.0f * kSlack - 1.0f) * qn;
+  float stagePart = queryPart, thrA = 0.0f;
+  const auto set_threshold = [&]() { thrA = fmaf(thr, (1.0f + kSlack) * s.scale2, stagePart); };
   const auto offer = [&](const Rec<float, D>& r) {
     const float d = dist2_seq(q, r);
     if (d <= thr && d <= maxRadius2 && heap.accepts(d, r.p.idx) && d > minDist) {
@@ -340,6 +377,14 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
     }
   };
 
+  // A stage's P. Its copy has been complete since before its first product,
+  // which the caller has read; the wait makes the copy visible to this thread,
+  // the records too.
+  const auto stage_bound = [&](int st, uint32_t round) {
+    mbar_wait(full(st), round, kTcDrainPolls);
+    return *reinterpret_cast<const float*>(smB + st * S::kB + S::kCopy - 16);
+  };
+
   bool ok = polls > 0;
   if (warp == 4) {
     if (lane == 0) {
@@ -347,8 +392,8 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
         const int64_t p = point_of(g);
         const int m = last - p < S::kStagePoints ? (int)(last - p) : S::kStagePoints;
         const uint32_t recBytes = (uint32_t)m * sizeof(Rec<float, D>);
-        mbar_expect(full(st), S::kB + recBytes);
-        bulk_load(smem_addr(smB + st * S::kB), operand + tc_offset<D>(p, 0), S::kB, full(st));
+        mbar_expect(full(st), S::kCopy + recBytes);
+        bulk_load(smem_addr(smB + st * S::kB), operand + p / S::kStagePoints * S::kCopy, S::kCopy, full(st));
         bulk_load(smem_addr(smR + st * S::kStagePoints), recs + p, recBytes, full(st));
       };
       const uint64_t da = tc_descriptor(smem_addr(smA), kRowGroup);
@@ -398,9 +443,10 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
 #pragma unroll
       for (int g = 0; g < kSlots; ++g) slot[g] = __int_as_float(0x7f800000);
       int st = 0;
+      float P = 0.25f;  // of all seeds
+      // (a seed's stage is whole: at least kTcSeedStride - 1 more follow it)
       for (int g = 0; g < seeds && ok; ++g) {
-        // the last stage's padding would count as points
-        const bool whole = point_of(g) + S::kStagePoints <= last;
+        bool far = false;
 #pragma unroll 1
         for (int i = 0; i < S::kTiles; ++i) {
           const int buf = (g * S::kTiles + i) % kBuffers;
@@ -410,26 +456,33 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (i == 0) {
+            const float p = stage_bound(st, g / kTcStages & 1);
+            far = p < 0.0f;
+            P = fmaxf(P, fabsf(p));
+          }
 #pragma unroll
           for (int part = 0; part < kTcPoints / 32; ++part) {
             uint32_t v[32];
             tc_load32(row + buf * kTcPoints + 32 * part, v);
             tc_wait_load(v);
-            if (whole) {
-              // value j to slot (32 part + j) % kSlots, two at a time where two
-              // of the 32 share a slot
-              if constexpr (kSlots >= 32) {
+            if (far) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  const int sl = (32 * part + j) % kSlots;
-                  slot[sl] = fminf(slot[sl], __uint_as_float(v[j]));
-                }
-              } else {
+              for (int j = 0; j < 32; ++j) v[j] = v[j] == 0xff800000u ? 0x7f800000u : v[j];
+            }
+            // value j to slot (32 part + j) % kSlots, two at a time where two
+            // of the 32 share a slot
+            if constexpr (kSlots >= 32) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  const int x = j / kSlots * 2 * kSlots + j % kSlots;
-                  slot[j % kSlots] = min3(slot[j % kSlots], __uint_as_float(v[x]), __uint_as_float(v[x + kSlots]));
-                }
+              for (int j = 0; j < 32; ++j) {
+                const int sl = (32 * part + j) % kSlots;
+                slot[sl] = fminf(slot[sl], __uint_as_float(v[j]));
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int x = j / kSlots * 2 * kSlots + j % kSlots;
+                slot[j % kSlots] = min3(slot[j % kSlots], __uint_as_float(v[x]), __uint_as_float(v[x + kSlots]));
               }
             }
           }
@@ -446,7 +499,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
         int near = 0;
         float bound = __int_as_float(0x7f800000);
         const float selfMax = minDist < 0.0f ? -__int_as_float(0x7f800000)
-                                             : (minDist * s.scale2 - qn) + kSlack * (minDist * s.scale2 + 2.0f * (s.pointMax + qn));
+                                             : (minDist * s.scale2 - qn) + kSlack * (minDist * s.scale2 + 2.0f * (P + qn));
 #pragma unroll 1
         for (int i = 0; i < a.k + 1; ++i) {  // take the smallest out, k + 1 times
           bound = slot[0];
@@ -461,13 +514,12 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
             out = out || hit;
           }
         }
-        if (!always && near <= 1) {
+        if (near <= 1) {
           // s^2 e <= bound + |q'|^2 + slack, rounded up
-          const float e = (bound + qn) + kSlack * (fabsf(bound + qn) + 2.0f * (s.pointMax + qn));
+          const float e = (bound + qn) + kSlack * (fabsf(bound + qn) + 2.0f * (P + qn));
           const float seed = __fmul_ru(fmaxf(e, 0.0f) * (1.0f + 0x1p-20f), 1.0f / s.scale2);
           if (seed < cap || !(cap == cap)) cap = cap == cap ? seed : cap;
           thr = bf_threshold(heap.head(), cap);
-          set_threshold();
         }
       }
     }
@@ -485,6 +537,11 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (i == 0) {
+          stagePart = fmaf(2.0f * kSlack, fabsf(stage_bound(st, round)), queryPart);
+          set_threshold();
+          thrA = thr != thr ? -__int_as_float(0x7f800000) : thrA;
+        }
         // the columns that pass, 32 at a time, the next ones on their way
         // meanwhile (one copy of the exact test serves all of them: inlined
         // per 32 columns it overflowed the instruction cache)
@@ -530,11 +587,8 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
           if (left < 32) mask[part] &= left > 0 ? (1u << left) - 1u : 0u;
           any |= mask[part];
         }
+        const Rec<float, D>* const tile = smR + st * S::kStagePoints + i * kTcPoints;
         if (any) {
-          // complete since before the product just read: makes the copied
-          // records visible to this thread
-          mbar_wait(full(st), round, kTcDrainPolls);
-          const Rec<float, D>* const tile = smR + st * S::kStagePoints + i * kTcPoints;
           do {
             int part = 0;
             unsigned bits = mask[0];
@@ -575,14 +629,34 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
     for (int g = max(copiedStages - kTcStages, 0); g < copiedStages; ++g)
       mbar_wait(full(g % kTcStages), (g / kTcStages) & 1, kTcDrainPolls);
   }
-  if (failed && warp < 4) {  // a wait ran out: this block's queries without the pipeline
-    heap.init(a.k);
-    cap = maxRadius2;
-    thr = bf_threshold(heap.head(), cap);
-    for (int64_t p = first; p < last; ++p) {
-      Rec<float, D> r;
-      load_rec(recs, p, r);
-      offer(r);
+  const bool plain = failed || beyond;
+  if (warp < 4 && __any_sync(0xffffffffu, plain)) {
+    // without the pipeline: all of the block's queries after a wait ran out,
+    // otherwise those beyond the filter. 32 points at a time, a lane loading
+    // each, their distances taken before the exact test.
+    if (plain) {
+      heap.init(a.k);
+      cap = maxRadius2;
+      thr = bf_threshold(heap.head(), cap);
+    }
+    for (int64_t base = first; base < last; base += 32) {
+      Rec<float, D> mine;
+      load_rec(recs, base + lane < last ? base + lane : last - 1, mine);
+      unsigned near = 0u;
+#pragma unroll 2
+      for (int j = 0; j < 32; ++j) {
+        Rec<float, D> r;
+#pragma unroll
+        for (int d = 0; d < D; ++d) r.p.c[d] = __shfl_sync(0xffffffffu, mine.p.c[d], j);
+        near |= base + j < last && dist2_seq(q, r) <= thr ? 1u << j : 0u;
+      }
+      while (plain && near) {
+        Rec<float, D> r;
+        load_rec(recs, base + __ffs(near) - 1, r);
+        near &= near - 1;
+        offer(r);
+      }
+      __syncwarp();
     }
   }
   __syncwarp();

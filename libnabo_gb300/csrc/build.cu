@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <limits>
 #include <vector>
@@ -168,12 +169,30 @@ __global__ void k_bounds(const Rec<T, D>* __restrict__ recs, int64_t n, int dim,
   }
 }
 
-template <typename T>
-__global__ void k_init_keys(typename KeyOf<T>::type* mnK, typename KeyOf<T>::type* mxK, int dim) {
-  const int d = threadIdx.x;
-  if (d < dim) {
-    mnK[d] = ordered_key(Ar<T>::inf());
-    mxK[d] = ordered_key(-Ar<T>::inf());
+// What a packed cloud's creation reads back, in one copy: the bounds' keys, a
+// flag for non-finite points, and a few points of a float cloud, evenly spread
+// but at irregular positions (a scan repeats itself every so many points).
+constexpr int kSamplePoints = 256;
+template <typename T, int D>
+struct CloudStats {
+  typename KeyOf<T>::type mn[kMaxDim], mx[kMaxDim];
+  int nonFinite;
+  T sample[sizeof(T) == 4 ? kSamplePoints : 1][D];
+};
+template <typename T, int D>
+__global__ void k_init_stats(CloudStats<T, D>* s, const Rec<T, D>* __restrict__ recs, int64_t n) {
+  const int i = threadIdx.x;
+  if (i < kMaxDim) {
+    s->mn[i] = ordered_key(Ar<T>::inf());
+    s->mx[i] = ordered_key(-Ar<T>::inf());
+  }
+  if (i == 0) s->nonFinite = 0;
+  if constexpr (sizeof(T) == 4) {
+    const int64_t first = n * i / kSamplePoints, width = n * (i + 1) / kSamplePoints - first;
+    int64_t p = first + (width > 0 ? (int64_t)((uint32_t)i * 2654435761u) % width : 0);
+    p = p < n ? p : n - 1;
+#pragma unroll
+    for (int d = 0; d < D; ++d) s->sample[i][d] = recs[p].p.c[d];
   }
 }
 
@@ -1005,32 +1024,56 @@ double host_key_to_double<double>(unsigned long long k) {
   return f;
 }
 
+// Centre and scale of the tensor-core filter's coordinates: the sample's medians,
+// and the power of 2 that brings all but its few farthest points to between 4
+// and 8 from there. Left at scale 0 when the cloud's range does not suit it.
+template <int D>
+void tc_scale(const CloudStats<float, D>& st, int dim, const double* lo, const double* hi, TcScale* s) {
+  constexpr int kFar = kSamplePoints / 32;
+  double widest = 0.0;
+  for (int d = 0; d < dim; ++d) {
+    if (!(std::fabs(lo[d]) < 1e15 && std::fabs(hi[d]) < 1e15)) return;
+    widest = std::max(widest, hi[d] - lo[d]);
+  }
+  if (!(widest > 1e-15)) return;
+  float v[kSamplePoints], reach[kSamplePoints] = {};
+  for (int d = 0; d < dim; ++d) {
+    for (int i = 0; i < kSamplePoints; ++i) v[i] = st.sample[i][d];
+    std::nth_element(v, v + kSamplePoints / 2, v + kSamplePoints);
+    s->centre[d] = v[kSamplePoints / 2];
+    for (int i = 0; i < kSamplePoints; ++i)
+      reach[i] = std::max(reach[i], std::fabs(st.sample[i][d] - s->centre[d]));
+  }
+  std::nth_element(reach, reach + kSamplePoints - 1 - kFar, reach + kSamplePoints);
+  double r = reach[kSamplePoints - 1 - kFar];
+  if (!(r > 1e-15)) r = widest;  // (nearly all points are one)
+  int e = 0;
+  std::frexp(r, &e);  // r <= 2^e
+  s->scale = (float)std::ldexp(1.0, 3 - e);
+  s->scale2 = s->scale * s->scale;
+}
+
 // Per-dimension bounds; fails on NaN or infinite coordinates, for which
 // the reference's split loop does not terminate (idealCutVal becomes NaN
 // and leftCount 0, nabo/kdtree_cpu.cpp:180-190).
 template <typename T, int D>
 int compute_bounds(const Rec<T, D>* recs, int64_t n, int dim, cudaStream_t stream, Scratch& sc, double* lo,
-                   double* hi) {
-  using Key = typename KeyOf<T>::type;
-  Key* keys;
-  int* flag;
-  NABO_CUDA_TRY(sc.get(&keys, 2 * kMaxDim));
-  NABO_CUDA_TRY(sc.get(&flag, 1));
-  NABO_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), stream));
-  k_init_keys<T><<<1, kMaxDim, 0, stream>>>(keys, keys + kMaxDim, dim);
+                   double* hi, TcScale* tc) {
+  CloudStats<T, D>* st;
+  NABO_CUDA_TRY(sc.get(&st, 1));
+  k_init_stats<T, D><<<1, kSamplePoints, 0, stream>>>(st, recs, n);
   const int grid = (int)std::min<int64_t>(ceil_div(n, kBlock), 152 * 8);
-  k_bounds<T, D><<<grid, kBlock, 0, stream>>>(recs, n, dim, keys, keys + kMaxDim, flag);
+  k_bounds<T, D><<<grid, kBlock, 0, stream>>>(recs, n, dim, st->mn, st->mx, &st->nonFinite);
   NABO_CUDA_TRY(cudaGetLastError());
-  Key h[2 * kMaxDim];
-  int hflag = 0;
-  NABO_CUDA_TRY(cudaMemcpyAsync(h, keys, sizeof(h), cudaMemcpyDeviceToHost, stream));
-  NABO_CUDA_TRY(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  CloudStats<T, D> h;
+  NABO_CUDA_TRY(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, stream));
   NABO_CUDA_TRY(cudaStreamSynchronize(stream));
-  if (hflag) return set_error(kErrArgument, "Cloud has non-finite (NaN or infinite) coordinates");
+  if (h.nonFinite) return set_error(kErrArgument, "Cloud has non-finite (NaN or infinite) coordinates");
   for (int d = 0; d < kMaxDim; ++d) {
-    lo[d] = d < dim ? host_key_to_double<T>(h[d]) : 0.0;
-    hi[d] = d < dim ? host_key_to_double<T>(h[kMaxDim + d]) : 0.0;
+    lo[d] = d < dim ? host_key_to_double<T>(h.mn[d]) : 0.0;
+    hi[d] = d < dim ? host_key_to_double<T>(h.mx[d]) : 0.0;
   }
+  if constexpr (sizeof(T) == 4) tc_scale<D>(h, dim, lo, hi, tc);
   return kOk;
 }
 
@@ -1044,7 +1087,7 @@ int pack_cloud(const T* dCloud, int64_t n, int64_t stride, int dim, cudaStream_t
   k_pack<T, D><<<ceil_div(n, kBlock), kBlock, 0, stream>>>(dCloud, n, stride, dim, recs);
   NABO_CUDA_TRY(cudaGetLastError());
   Scratch sc(stream);
-  const int rc = compute_bounds<T, D>(recs, n, dim, stream, sc, out->lo, out->hi);
+  const int rc = compute_bounds<T, D>(recs, n, dim, stream, sc, out->lo, out->hi, &out->tc);
   if (rc != kOk) return rc;
   return kOk;
 }

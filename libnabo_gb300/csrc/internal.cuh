@@ -86,13 +86,11 @@ void set_capture_allocations(bool on);
 // Whether a caller (not the library itself) is capturing the stream.
 bool caller_captures(cudaStream_t stream);
 
-// Coordinates of the tensor-core brute force (bruteforce_tc.cuh): s (x - c),
-// with P at least every point's squared norm.
+// Coordinates of the tensor-core brute force (bruteforce_tc.cuh): s (x - c).
 struct TcScale {
   float centre[kMaxDim];
-  float scale;    // s, a power of 2
-  float scale2;   // s^2
-  float pointMax; // P
+  float scale;   // s, a power of 2; 0: the cloud does not suit it
+  float scale2;  // s^2
 };
 
 // Device-resident kd-tree (or, for brute force, the packed cloud only).
@@ -113,10 +111,10 @@ struct DeviceCloud {
   // coordinate magnitude (device float), for the search's float pre-filter
   void* recs32 = nullptr;
   float* coordMax = nullptr;
-  // float brute force: the points as the tensor cores' operand and its
-  // coordinates (prepare_bruteforce), or null
-  void* tcOperand = nullptr;
+  // float brute force: the tensor cores' coordinates (pack_cloud) and the
+  // points as their operand (prepare_bruteforce), or null
   TcScale tc = {};
+  void* tcOperand = nullptr;
 };
 
 struct BuildStats {

@@ -8,7 +8,6 @@
 #include "search_wide.cuh"
 
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 #include <string>
 
@@ -372,29 +371,6 @@ int launch_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
   return kOk;
 }
 
-// Centre and scale of the tensor-core filter's coordinates; false when the
-// cloud's range does not suit it.
-inline bool tc_scale(const DeviceCloud& c, TcScale* s) {
-  double half[kMaxDim], widest = 0.0;
-  for (int d = 0; d < kMaxDim; ++d) {
-    s->centre[d] = 0.0f;
-    if (d >= c.dim) continue;
-    if (!(std::fabs(c.lo[d]) < 1e15 && std::fabs(c.hi[d]) < 1e15)) return false;
-    s->centre[d] = (float)(0.5 * (c.lo[d] + c.hi[d]));
-    half[d] = std::max(c.hi[d] - (double)s->centre[d], (double)s->centre[d] - c.lo[d]);
-    widest = std::max(widest, half[d]);
-  }
-  if (!(widest > 1e-15)) return false;
-  int e = 0;
-  std::frexp(widest, &e);  // widest <= 2^e
-  s->scale = (float)std::ldexp(1.0, -e);
-  s->scale2 = s->scale * s->scale;
-  double p = 0.0;
-  for (int d = 0; d < c.dim; ++d) p += half[d] * half[d] * s->scale2;
-  s->pointMax = (float)std::max(0.25, p * (1.0 + 1e-5));
-  return true;
-}
-
 // Block rows (parts of the points) of a search of qBlocks query blocks when
 // `slots` blocks run at once: fewest waves per row (the last, partly empty one
 // counted as 0.4 of one more), each further row costing 4 + k percent (at
@@ -461,16 +437,15 @@ constexpr int64_t kTcMinPoints = 512;
 template <typename T, int D>
 int prepare_bruteforce(DeviceCloud& c, cudaStream_t stream) {
   if constexpr (sizeof(T) == 4) {
-    if (c.n < kTcMinPoints || !tc_scale(c, &c.tc)) return kOk;
-    constexpr int kStage = TcSmem<D, 1>::kStagePoints;
-    const int64_t padded = (c.n + kStage - 1) / kStage * kStage;
-    if (object_alloc(&c.tcOperand, TcShape<D>::operandBytes(1) * (size_t)padded, stream) != cudaSuccess) {
+    if (c.n < kTcMinPoints || !(c.tc.scale > 0.0f)) return kOk;
+    const int64_t stages = (c.n + TcStage<D>::kPoints - 1) / TcStage<D>::kPoints;
+    if (object_alloc(&c.tcOperand, (size_t)stages * TcStage<D>::kBytes, stream) != cudaSuccess) {
       cudaGetLastError();
       c.tcOperand = nullptr;
       return kOk;
     }
-    k_bf_tc_points<D><<<ceil_div(padded, 256), 256, 0, stream>>>(static_cast<const Rec<float, D>*>(c.recs), c.n, padded,
-                                                                 c.dim, c.tc, static_cast<unsigned char*>(c.tcOperand));
+    k_bf_tc_points<D><<<(unsigned)stages, TcStage<D>::kPoints, 0, stream>>>(
+        static_cast<const Rec<float, D>*>(c.recs), c.n, c.dim, c.tc, static_cast<unsigned char*>(c.tcOperand));
     NABO_CUDA_TRY(cudaGetLastError());
   }
   return kOk;
