@@ -1136,15 +1136,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   int midOcc = 0;
   NABO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&midOcc, k_mid<T, D>, Mid::kThreads, midSmem));
 
-  // k_top: one block per SM, each with its share of the positions
   const bool top = !median && n > smallMax;
-  const int chunk = (int)std::max<int64_t>(kTopMinChunk, ((n + sms - 1) / sms + 31) / 32 * 32);
-  const int topBlocks = ceil_div(n, chunk);
-  // the segments overlapping a chunk hold more than smallMax points each
-  const int pieces = chunk / smallMax + 2;
-  const size_t withRecs = TopShape<T, D>::bytes(chunk, pieces, true);
-  const size_t withLists = TopShape<T, D>::bytes(chunk, pieces, false);
-  const int topMode = withRecs <= kTopSmemMax ? kTopResident : (withLists <= kTopSmemMax ? kTopLists : kTopGlobal);
 
   const int64_t segCap = n / (smallMax + 1) + 2;
   const int64_t smallCap = n / ((int64_t)bucket + 1) + nClouds + 2;
@@ -1195,11 +1187,10 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
       take_level(A, nxt, segCap);
     } else if (top) {
       A.take(ta.exch, n);
-      if (topMode == kTopGlobal) A.take(ta.work, (int64_t)withLists * topBlocks);
-      A.take(ta.head, topBlocks);
-      A.take(ta.tail, topBlocks);
-      A.take(ta.head2, topBlocks);
-      A.take(ta.tail2, topBlocks);
+      A.take(ta.head, sms);
+      A.take(ta.tail, sms);
+      A.take(ta.head2, sms);
+      A.take(ta.tail2, sms);
     }
   };
   Arena A;
@@ -1245,23 +1236,44 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
     ta.n = N;
     ta.nClouds = nClouds;
     ta.dim = dim;
-    ta.chunk = chunk;
-    ta.pieces = pieces;
     ta.smallMax = smallMax;
     ta.bucket = bucket;
     ta.maxLevels = maxLevels;
     ta.smallCap = (int)smallCap;
     ta.barrierPolls = f->barrierPolls;
-    ta.workBytes = (int64_t)withLists;
-    const void* kernel = topMode == kTopResident ? (const void*)k_top<T, D, kTopResident>
-                         : topMode == kTopLists  ? (const void*)k_top<T, D, kTopLists>
-                                                 : (const void*)k_top<T, D, kTopGlobal>;
-    const size_t topSmem = topMode == kTopResident ? withRecs : (topMode == kTopLists ? withLists : 0);
-    // the most any build asks for, as k_mid's
-    if (topSmem > 0)
-      NABO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmemMax));
-    void* args[] = {&ta};
-    NABO_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(topBlocks), dim3(kTopThreads), args, topSmem, stream));
+    // One block per SM, each with its share of the positions. All of them have
+    // to be resident at once: where the launch may use fewer SMs than the
+    // device has (a stream or context with a part of them) it is refused, and
+    // fewer blocks take more positions each.
+    for (int most = sms;;) {
+      const int chunk = (int)std::max<int64_t>(kTopMinChunk, ((n + most - 1) / most + 31) / 32 * 32);
+      const int topBlocks = ceil_div(n, chunk);
+      // the segments overlapping a chunk hold more than smallMax points each
+      const int pieces = chunk / smallMax + 2;
+      const size_t withRecs = TopShape<T, D>::bytes(chunk, pieces, true);
+      const size_t withLists = TopShape<T, D>::bytes(chunk, pieces, false);
+      const int topMode = withRecs <= kTopSmemMax ? kTopResident : (withLists <= kTopSmemMax ? kTopLists : kTopGlobal);
+      ta.chunk = chunk;
+      ta.pieces = pieces;
+      ta.workBytes = (int64_t)withLists;
+      if (topMode == kTopGlobal) NABO_CUDA_TRY(sc.get(&ta.work, (int64_t)withLists * topBlocks));
+      const void* kernel = topMode == kTopResident ? (const void*)k_top<T, D, kTopResident>
+                           : topMode == kTopLists  ? (const void*)k_top<T, D, kTopLists>
+                                                   : (const void*)k_top<T, D, kTopGlobal>;
+      const size_t topSmem = topMode == kTopResident ? withRecs : (topMode == kTopLists ? withLists : 0);
+      // the most any build asks for, as k_mid's
+      if (topSmem > 0)
+        NABO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmemMax));
+      void* args[] = {&ta};
+      const cudaError_t e =
+          cudaLaunchCooperativeKernel(kernel, dim3(topBlocks), dim3(kTopThreads), args, topSmem, stream);
+      if (e != cudaErrorCooperativeLaunchTooLarge || topBlocks == 1) {
+        NABO_CUDA_TRY(e);
+        break;
+      }
+      cudaGetLastError();
+      most = topBlocks / 2;
+    }
   }
   if (median) {
     if (nPad > 0) {

@@ -11,14 +11,14 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def compile_cu(tmp_path, name):
+def compile_cu(tmp_path, name, *extra):
     from libnabo_gb300 import build
     lib = os.path.join(ROOT, "libnabo_gb300", "lib")
     exe = str(tmp_path / name)
     subprocess.run([build.nvcc(), *build.ARCH, "-O1", "-std=c++17", "-Xcompiler", "-ffp-contract=off",
                     "-I", os.path.join(ROOT, "include"), "-I", build.CSRC, os.path.join(ROOT, "tests", "cpp", f"{name}.cu"),
                     "-L", lib, "-lnabo_gb300", "-Xlinker", f"-rpath={lib}", "-Xlinker", "--export-dynamic", "-ldl",
-                    "-o", exe], check=True, capture_output=True, text=True)
+                    *extra, "-o", exe], check=True, capture_output=True, text=True)
     return exe
 
 
