@@ -93,6 +93,13 @@ struct TcScale {
   float scale2;  // s^2
 };
 
+// SMs of the current device.
+inline int sm_count() {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 // Device-resident kd-tree (or, for brute force, the packed cloud only).
 struct DeviceCloud {
   int dtype = 0;        // 0 = f32, 1 = f64

@@ -885,7 +885,7 @@ int launch_radius(const RadiusModel& m, const void* query, int64_t nq, int64_t q
   ro.margin = m.margin;
   ro.maxRadius = maxRadius;
   const int64_t tiles = (nq + 15) / 16;
-  const int grid = (int)std::min<int64_t>(ceil_div(tiles, kInferWarps), 152 * kInferBlocks);
+  const int grid = (int)std::min<int64_t>(ceil_div(tiles, kInferWarps), (int64_t)sm_count() * kInferBlocks);
   if (m.dtype == NABO_CUDA_FLOAT32)
     k_mlp_radius<float><<<grid, kInferWarps * 32, 0, st>>>(static_cast<const float*>(query), nq, qStride, m.fs, m.pb,
                                                              ro, static_cast<float*>(radii), raw);

@@ -140,12 +140,6 @@ int launch_wide_bruteforce(const KnnLaunch& L, cudaStream_t stream) {
   return k_unsupported();
 }
 
-inline int sm_count() {
-  int dev = 0, sms = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Queries per warp of the one-thread-per-query search. A warp takes as long as
 // its lanes' paths together where they diverge, so a search too small to fill
 // the GPU runs fewer queries in each of more warps: the fewest lanes (a power
