@@ -280,29 +280,24 @@ __device__ __forceinline__ int arg_max_extent(const T* lo, const T* hi, int dim)
 // exact up to kHeld points, in k_mid). Just above (the next representable
 // value): points equal to the median go left and hardly any lies on the cut.
 
-// Single block: exclusive scan of the per-block sums; the grand total goes
-// to *total. Each thread scans a contiguous run serially and one block-wide
+// Single block: exclusive scan of the per-block sums. Each thread scans a contiguous run serially and one block-wide
 // scan joins the runs (a loop of block-wide scans over the sums would
 // serialise on its barriers: 0.2 ms per call at 22 M points).
-__global__ void k_scan_block_sums(int2* sums, int nb, int2* total, const LevelState* st) {
+__global__ void k_scan_block_sums(int2* sums, int nb, const LevelState* st) {
   pdl_begin();
-  if (st->nseg == 0) {
-    if (threadIdx.x == 0) *total = make_int2(0, 0);
-    return;
-  }
+  if (st->nseg == 0) return;
   const int per = (nb + kBlock - 1) / kBlock;
   const int b0 = threadIdx.x * per;
   const int b1 = min(b0 + per, nb);
   int2 run = make_int2(0, 0);
   for (int i = b0; i < b1; ++i) run = add2(run, sums[i]);
-  int2 t;
-  int2 carry = block_excl_scan(run, &t);
+  int2 total;
+  int2 carry = block_excl_scan(run, &total);
   for (int i = b0; i < b1; ++i) {
     const int2 v = sums[i];
     sums[i] = carry;
     carry = add2(carry, v);
   }
-  if (threadIdx.x == 0) *total = t;
 }
 
 // Records the split of segment s of the current level and its two children,
@@ -390,9 +385,8 @@ __global__ void k_advance(LevelState* st, int* counters) {
 // reads. Segment ids and cut coordinates travel with the records, so a
 // level reads each position's id and coordinate twice and its record once,
 // and writes its record, next id and next coordinate once: 6 launches and
-// about 56 bytes per position of a large segment per level, against 14
-// launches for the reference's rule. The arrays in use alternate with the
-// level's parity (LevelState::level), read on the device, so a fixed-level
+// about 56 bytes per position of a large segment per level. The arrays in use
+// alternate with the level's parity (LevelState::level), read on the device, so a fixed-level
 // build needs no host decision.
 constexpr int kItems = 4;               // consecutive positions per thread
 constexpr int kTile = kBlock * kItems;  // positions per block and tile
@@ -424,14 +418,6 @@ __device__ __forceinline__ void load4(const T* __restrict__ p, T (&v)[kItems]) {
     v[2] = b.x;
     v[3] = b.y;
   }
-}
-
-template <typename T, int D>
-__device__ __forceinline__ T rec_coord(const Rec<T, D>& r, int cd) {
-  T v = r.p.c[0];
-#pragma unroll
-  for (int d = 1; d < D; ++d) v = d == cd ? r.p.c[d] : v;
-  return v;
 }
 
 // One tile's positions of a thread: segment ids, coordinates and the two
@@ -489,7 +475,7 @@ __global__ void k_median_cut(SegLevel<T> L, const LevelState* st, MedianBufs<T, 
 
 // Block b scans tiles [b * tiles, (b + 1) * tiles) in position order and
 // records, besides its totals, each segment's running flag counts at its
-// first position (exclusive) and last position (inclusive), as k_flag_sums.
+// first position (exclusive) and last position (inclusive).
 // The next tile's ids and coordinates are loaded before this tile's scan.
 template <typename T, int D>
 __global__ void k_median_sums(MedianBufs<T, D> B, int64_t nPad, SegLevel<T> L, int tiles, int2* blockSums,
@@ -638,7 +624,7 @@ __global__ void k_median_scatter(MedianBufs<T, D> B, Rec<T, D>* __restrict__ fin
         if (child >= 0) {
           dst[dest] = r;
           segN[dest] = child;
-          valN[dest] = rec_coord(r, next.cutDim[child]);
+          valN[dest] = coord_of(r, next.cutDim[child]);
         } else {
           finalRecs[dest] = r;
           segN[dest] = -1;
@@ -744,7 +730,7 @@ __global__ void k_median_scatter_staged(MedianBufs<T, D> B, Rec<T, D>* __restric
       sRec[j] = r;
       sChild[j] = child;
       sDest[j] = dest[i];
-      if (child >= 0) sVal[j] = rec_coord(r, next.cutDim[child]);
+      if (child >= 0) sVal[j] = coord_of(r, next.cutDim[child]);
     }
     __syncthreads();
     const int moved = sideTotal.x + sideTotal.y;
@@ -1152,7 +1138,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
   SegList<T> small;
   MedianBufs<T, D> mb = {};
   int* rootSeg = nullptr;
-  int2 *passTotal, *blockSums, *segFirst, *segLast;
+  int2 *blockSums, *segFirst, *segLast;
   SegLevel<T> cur = {}, nxt = {};
   TopArgs<T, D> ta = {};
   size_t zeroed = 0;
@@ -1179,7 +1165,6 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
         A.take(mb.val[i], nPad);
       }
       A.take(rootSeg, nClouds);
-      A.take(passTotal, 1);
       A.take(blockSums, nb);
       A.take(segFirst, segCap);
       A.take(segLast, segCap);
@@ -1302,7 +1287,7 @@ int build_forest(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
       NABO_CUDA_TRY(launch_pdl(k_median_cut<T, D>, ceil_div(segCap, 4), 128, 0, stream, cur, st, mb));
       NABO_CUDA_TRY(launch_pdl(k_median_sums<T, D>, mBlocks, kBlock, 0, stream, mb, nPad, cur, mTiles, blockSums,
                                segFirst, segLast, st));
-      NABO_CUDA_TRY(launch_pdl(k_scan_block_sums, 1, kBlock, 0, stream, blockSums, mBlocks, passTotal, st));
+      NABO_CUDA_TRY(launch_pdl(k_scan_block_sums, 1, kBlock, 0, stream, blockSums, mBlocks, st));
       NABO_CUDA_TRY(launch_pdl(k_median_split<T, D>, sg, 128, 0, stream, cur, nxt, st, small, marks, counters, dim,
                                bucket, smallMax, (int)segCap, (int)smallCap, (const int2*)blockSums, (const int2*)segFirst,
                                (const int2*)segLast, mTiles * kTile));
@@ -1359,7 +1344,7 @@ __global__ void k_one_cloud(BuildResult<T>* r, int64_t n) {
 
 template <typename T, int D>
 int build_kdtree(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned bucketSize, cudaStream_t stream,
-                 DeviceCloud* out, double* rootMin, double* rootMax, BuildStats* stats, int splitRule) {
+                 DeviceCloud* out, double* rootMin, double* rootMax, int splitRule) {
   Scratch sc(stream);
   ForestOut f;
   Rec<T, D>* recs = nullptr;
@@ -1403,9 +1388,6 @@ int build_kdtree(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned b
     // unless the quirk lifted it to numeric_limits<T>::min()
     out->lo[d] = rootMin[d];
     out->hi[d] = rootMax[d];
-  }
-  if (stats) {
-    stats->topLevels = hs[3];
   }
   return kOk;
 }
@@ -1461,7 +1443,7 @@ template int narrow_records<16>(const void*, int64_t, int, void*, float*, cudaSt
 
 #define NABO_BUILD_INSTANTIATE(T, D)                                                                          \
   template int build_kdtree<T, D>(const T*, int64_t, int64_t, int, unsigned, cudaStream_t, DeviceCloud*,      \
-                                  double*, double*, BuildStats*, int);                                        \
+                                  double*, double*, int);                                                      \
   template int build_forest<T, D>(const T*, int64_t, int64_t, int, unsigned, const int64_t*, int, int,        \
                                   cudaStream_t, ForestOut*, int);                                             \
   template int pack_cloud<T, D>(const T*, int64_t, int64_t, int, cudaStream_t, DeviceCloud*);

@@ -409,7 +409,7 @@ int build_any(nabo_cuda_search* h, const void* dCloud, int64_t stride, cudaStrea
     int rc = kOk;
     NABO_DISPATCH_RC(rc, h->c.dtype, h->c.dpad,
                      (build_kdtree<T, D>(static_cast<const T*>(dCloud), h->c.n, stride, h->c.dim, h->c.bucketSize,
-                                         st, &h->c, rootMin, rootMax, nullptr, h->c.splitRule)));
+                                         st, &h->c, rootMin, rootMax, h->c.splitRule)));
     if (rc == kOk && h->c.dtype == NABO_CUDA_FLOAT64) rc = narrow_cloud(h->c, st);
     return rc;
   }

@@ -124,10 +124,6 @@ struct DeviceCloud {
   void* tcOperand = nullptr;
 };
 
-struct BuildStats {
-  int topLevels = 0;  // levels split before the small segments' phase
-};
-
 // Builds the kd-tree of `n` points (dim coordinates each, column stride
 // `stride` elements) held in device memory at `dCloud`. Produces the same
 // tree as the reference's KDTreeUnbalancedPtInLeavesImplicitBoundsStackOpt
@@ -138,7 +134,7 @@ struct BuildStats {
 // balanced tree, not the reference's; see nabo_cuda_params::splitRule).
 template <typename T, int D>
 int build_kdtree(const T* dCloud, int64_t n, int64_t stride, int dim, unsigned bucketSize, cudaStream_t stream,
-                 DeviceCloud* out, double* rootMin, double* rootMax, BuildStats* stats, int splitRule = 0);
+                 DeviceCloud* out, double* rootMin, double* rootMax, int splitRule = 0);
 
 // Output buffers of a forest build (all device memory, allocated by the
 // caller): records (n), nodes (2n), nodeOffset (nClouds+1), root boxes
@@ -294,12 +290,13 @@ struct KnnArgs {
   int waitPolls = 1 << 22;
 };
 
-// Whether a search runs its queries in a sorted order. The sort costs about
-// 130 us almost whatever the size, so it pays only for enough work: measured
-// on GB300, 3-D lidar scans at k = 10 gained from 2^18 queries (440 vs
-// 470 us) and lost below (131 k: 346 vs 260 us), while 8-D clustered clouds
-// at k = 32 gained 30 % at 200 k queries (16.7 vs 23.9 ms). The rule weighs
-// the queries by k and by the dimension.
+// Whether a search runs its queries in a sorted order. The sort pays only for
+// enough work: measured on GB300 when it took about 130 us almost whatever the
+// size, 3-D lidar scans at k = 10 gained from 2^18 queries (440 vs 470 us) and
+// lost below (131 k: 346 vs 260 us), while 8-D clustered clouds at k = 32
+// gained 30 % at 200 k queries (16.7 vs 23.9 ms). The rule weighs the queries
+// by k and by the dimension. (The sort now takes 94 us of kernels at 1.15 M
+// queries; the line has not been measured again.)
 inline bool worth_sorting(int64_t nq, int k, int dim) {
   const double work = (double)nq * (k + 10) / 20.0 * (dim > 3 ? 8.0 : 1.0);
   return work >= (double)(int64_t(1) << 18);

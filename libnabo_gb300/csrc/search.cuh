@@ -533,15 +533,11 @@ __device__ __forceinline__ void scan_leaf(const Rec<T, D>* __restrict__ recs, ui
   for (uint32_t base = 0; base < cnt; base += kChunk) {
     unsigned mask = 0;
     if constexpr (std::is_same<T, float>::value) {
-      // float: candidates as packed (dist2 bits, index) keys, one 64-bit
-      // compare against min(head, radius key) -- the radius key is the
-      // largest key of distance maxRadius2, so d <= maxRadius2 && key <
-      // head is key < that minimum (a NaN radius accepts nothing: 0) --
-      // and one 64-bit select per insertion (4-9 % faster than separate
-      // radius and head tests on lidar scans)
-      const uint64_t radKey = maxRadius2 == maxRadius2 ? ((uint64_t(__float_as_uint(maxRadius2)) << 32) | 0xffffffffull) : 0ull;
-      const uint64_t thrKey =
-          (!want || radKey == 0ull) ? 0ull : (heap.key[0] <= radKey ? heap.key[0] : radKey + 1ull);
+      // float: one float compare against min(head, maxRadius2) lets a
+      // candidate pass (NaN: none), and its packed (dist2 bits, index) key
+      // decides ties with the head where it is inserted (1.15 M lidar
+      // points, k = 10: 1036 us, against 1053 with the keys compared for
+      // every point)
       uint64_t kj[kChunk];
       const float hd = heap.head();
       const float thrF = want ? (hd < maxRadius2 ? hd : maxRadius2) : __int_as_float(0x7fffffff);
