@@ -22,20 +22,21 @@
 struct Tree {
   std::vector<uint32_t> right, start, count;
   std::vector<int32_t> cutDim, buckets;
-  std::vector<float> cut;
+  std::vector<double> cut;
   bool operator==(const Tree& o) const {
     return right == o.right && start == o.start && count == o.count && cutDim == o.cutDim && buckets == o.buckets &&
            cut == o.cut;
   }
 };
 
-static Tree build(const std::vector<float>& cloud, cudaStream_t st) {
-  const int64_t n = (int64_t)cloud.size() / 3;
-  float* d;
-  CHECK(cudaMalloc(&d, cloud.size() * 4) == cudaSuccess);
-  CHECK(cudaMemcpy(d, cloud.data(), cloud.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess);
+template <typename T>
+static Tree build(const std::vector<T>& cloud, int dim, cudaStream_t st) {
+  const int64_t n = (int64_t)cloud.size() / dim;
+  T* d;
+  CHECK(cudaMalloc(&d, cloud.size() * sizeof(T)) == cudaSuccess);
+  CHECK(cudaMemcpy(d, cloud.data(), cloud.size() * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess);
   nabo_cuda_batch* b = nullptr;
-  CHECK(nabo_cuda_batch_create(NABO_CUDA_FLOAT32, 3, 1, &n, nullptr, 0, &b) == 0);
+  CHECK(nabo_cuda_batch_create(sizeof(T) == 4 ? NABO_CUDA_FLOAT32 : NABO_CUDA_FLOAT64, dim, 1, &n, nullptr, 0, &b) == 0);
   CHECK(nabo_cuda_batch_build_device(b, d, st) == 0);
   CHECK(cudaStreamSynchronize(st) == cudaSuccess);
   int64_t status[8], nodes = 0;
@@ -46,18 +47,30 @@ static Tree build(const std::vector<float>& cloud, cudaStream_t st) {
   t.start.resize(nodes);
   t.count.resize(nodes);
   t.cutDim.resize(nodes);
-  t.cut.resize(nodes);
+  std::vector<T> cut(nodes);
   t.buckets.resize(n);
-  CHECK(nabo_cuda_batch_export_tree(b, 0, &nodes, t.cutDim.data(), t.cut.data(), t.right.data(), t.start.data(),
+  CHECK(nabo_cuda_batch_export_tree(b, 0, &nodes, t.cutDim.data(), cut.data(), t.right.data(), t.start.data(),
                                     t.count.data(), t.buckets.data()) == 0);
+  t.cut.assign(cut.begin(), cut.end());
   CHECK(nabo_cuda_batch_destroy(b) == 0);
   CHECK(cudaFree(d) == cudaSuccess);
   return t;
 }
 
-int main() {
+template <typename T>
+static void check(int64_t n, int dim, cudaStream_t st) {
   std::mt19937 rng(3);
-  std::uniform_real_distribution<float> u(0.0f, 1.0f);
+  std::uniform_real_distribution<T> u(0, 1);
+  std::vector<T> c(n * dim);
+  for (T& x : c) x = u(rng);
+  for (int64_t i = 0; i < n; i += 5) c[i * dim] = T(0.5);  // points on a cut
+  const Tree want = build(c, dim, nullptr);
+  CHECK(want.right.size() > 1);
+  CHECK(build(c, dim, st) == want);
+  std::printf("ok n=%lld D=%d\n", (long long)n, dim);
+}
+
+int main() {
   CHECK(cudaFree(nullptr) == cudaSuccess);
   CUdevResource all, part;
   unsigned groups = 1;
@@ -73,14 +86,9 @@ int main() {
     return 77;
   }
   std::printf("%u of %u SMs\n", part.sm.smCount, all.sm.smCount);
-  for (int64_t n : {3000, 20000, 90000, 1200000}) {
-    std::vector<float> c(n * 3);
-    for (float& x : c) x = u(rng);
-    const Tree want = build(c, nullptr);
-    CHECK(want.right.size() > 1);
-    CHECK(build(c, st) == want);
-    std::printf("ok n=%lld\n", (long long)n);
-  }
+  for (int64_t n : {3000, 20000, 90000, 1200000}) check<float>(n, 3, st);
+  // so many positions a block that its lists do not fit in shared memory
+  check<double>(2500000, 16, st);
   CHECK(cudaStreamDestroy(st) == cudaSuccess);
   CHECK(cuGreenCtxDestroy(green) == CUDA_SUCCESS);
 }

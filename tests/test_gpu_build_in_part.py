@@ -1,5 +1,6 @@
 """A build on a stream that may use some of the device's SMs only: the launch of the top levels, whose blocks all have to be
-resident, takes as many as the stream has room for (tests/cpp/build_in_part.cu)."""
+resident, takes as many as the stream has room for, and their working lists leave shared memory when they are too long for it
+(tests/cpp/build_in_part.cu)."""
 import os
 import subprocess
 
@@ -17,4 +18,4 @@ def test_green_context_stream(tmp_path):
                        timeout=300)
     if r.returncode == 77:
         pytest.skip("no green contexts here")
-    assert r.returncode == 0 and r.stdout.count("ok ") == 4, r.stdout + r.stderr
+    assert r.returncode == 0 and r.stdout.count("ok ") == 5, r.stdout + r.stderr
