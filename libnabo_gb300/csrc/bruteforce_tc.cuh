@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kTcThreads, TcTile<K>::kBlocksPerSm)
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       q[d] = active && d < a.dim ? static_cast<const float*>(a.query)[qi * a.qStride + d] : 0.0f;
-      x[d] = d < a.dim ? (q[d] - s.centre[d]) * s.scale : 0.0f;
+      x[d] = active && d < a.dim ? (q[d] - s.centre[d]) * s.scale : 0.0f;  // (an idle slot: within the range)
       qn = fmaf(x[d], x[d], qn);
       beyond = beyond || !(fabsf(x[d]) <= kTcQueryMax);
     }
